@@ -140,11 +140,21 @@ b200_status b200_context_create(int device_ordinal, b200_context** out) {
   if (e == cudaSuccess) e = cudaMalloc(&ctx->qtc_parts, ctx->qtc_parts_floats * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&ctx->qtc_counters, ctx->qtc_tiles_max * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(ctx->qtc_counters, 0, ctx->qtc_tiles_max * sizeof(unsigned));
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device_ordinal;
+    e = cudaMemPoolCreate(&ctx->pool, &props);
+    uint64_t keep = kPoolKeepBytes;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
   if (e != cudaSuccess) {
     b200_status s = Fail(B200_RESOURCE_EXHAUSTED, "context allocation: %s", cudaGetErrorString(e));
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->qtc_parts) cudaFree(ctx->qtc_parts);
     if (ctx->qtc_counters) cudaFree(ctx->qtc_counters);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
     return s;
   }
@@ -164,6 +174,7 @@ void b200_context_destroy(b200_context* ctx) {
   if (ctx->qtc_parts) cudaFree(ctx->qtc_parts);
   if (ctx->qtc_counters) cudaFree(ctx->qtc_counters);
   if (ctx->qmm_ws) cudaFree(ctx->qmm_ws);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->host_status) cudaFreeHost(ctx->host_status);
   delete ctx;
 }

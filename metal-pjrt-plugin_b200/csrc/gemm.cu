@@ -11,6 +11,8 @@
 //   few-row  - the bandwidth-bound streaming kernel (qmm.cu, 16-bit weights), for
 //              x . W^T with up to 32 rows on either side; preferred up to 8 rows, above
 //              that the tensor-core route (which splits K across a cluster) is faster;
+//              (operands whose rows are not 16-byte aligned are copied into aligned rows first,
+//              where the product is large enough to pay for the copy);
 //   SIMT     - the general tile kernel below: every dtype, transpose, stride,
 //              batch and beta; true f32 arithmetic for f32 operands (tensor
 //              cores have no f32 multiply, and the f32 block must hold rtol 1e-5).
@@ -27,6 +29,7 @@ b200_status RunFewRowNT(b200_context* ctx, cudaStream_t stream, const void* mat,
                         void* aux, int out_f32);
 // gemm_tcgen05.cu
 bool Tcgen05Supports(const b200_gemm_params* p, const b200_epilogue* epi);
+bool TmaReadable(const b200_operand& x, int64_t batch);
 b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_params* p, const b200_epilogue* epi);
 }  // namespace b200
 
@@ -140,6 +143,84 @@ cudaError_t LaunchSimt(const SimtArgs& a, int64_t batch, cudaStream_t stream) {
   return Launch(lc, gemm_simt_kernel<TIn, TOut>, a);
 }
 
+// Copies rows of `cols` 16-bit elements that start anywhere into rows of `dst_words` 32-bit words.  Bound by memory:
+// a warp moves 128 contiguous bytes; a row that starts on an odd element is put together from the two words around
+// each pair (the second comes from L1).
+__global__ void __launch_bounds__(256) align_rows_kernel(const uint16_t* src, uint32_t* dst, int64_t rows_per_batch, int64_t rows,
+                                                         int cols, int64_t ld, int64_t batch_stride, int dst_words) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int words = (cols + 1) / 2;
+  for (int64_t r = blockIdx.y * static_cast<int64_t>(blockDim.y) + threadIdx.y; r < rows; r += static_cast<int64_t>(gridDim.y) * blockDim.y) {
+    const uint16_t* s = src + (r / rows_per_batch) * batch_stride + (r % rows_per_batch) * ld;
+    uint32_t* d = dst + r * dst_words;
+    const bool odd = (reinterpret_cast<uintptr_t>(s) & 2) != 0;
+    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x) {
+      uint32_t v;
+      if (2 * w + 1 >= cols) v = __ldg(s + 2 * w);
+      else if (!odd) v = __ldg(reinterpret_cast<const uint32_t*>(s) + w);
+      else v = __byte_perm(__ldg(reinterpret_cast<const uint32_t*>(s - 1) + w), __ldg(reinterpret_cast<const uint32_t*>(s - 1) + w + 1), 0x5432);
+      d[w] = v;
+    }
+  }
+}
+
+b200_status AlignRows(b200_context* ctx, cudaStream_t stream, const b200_operand& x, int64_t rows, int64_t cols, int64_t batches,
+                      void* dst, int64_t dst_ld) {
+  b200_status s = BeginLaunch(ctx);
+  if (s != B200_OK) return s;
+  const int words = static_cast<int>(CeilDiv(cols, 2));
+  const int tx = words >= 128 ? 128 : 32, ty = 256 / tx;
+  LaunchCfg lc;
+  lc.block = dim3(tx, ty);
+  const int64_t all = rows * batches, gx = std::min<int64_t>(CeilDiv(words, 4 * tx), 64);
+  lc.grid = dim3(static_cast<unsigned>(std::max<int64_t>(gx, 1)), static_cast<unsigned>(std::min<int64_t>(CeilDiv(all, ty), std::max<int64_t>(1, ctx->sm_count * 16 / std::max<int64_t>(gx, 1)))));
+  lc.stream = stream;
+  lc.pdl = true;
+  cudaError_t e = Launch(lc, align_rows_kernel, static_cast<const uint16_t*>(x.ptr), static_cast<uint32_t*>(dst), rows, all,
+                         static_cast<int>(cols), x.ld, batches > 1 ? x.batch_stride : 0, static_cast<int>(dst_ld / 2));
+  if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_gemm: row alignment launch: %s", cudaGetErrorString(e)));
+  return EndLaunch(ctx, "b200_gemm (row alignment)");
+}
+
+// The same product with every operand that TMA cannot read copied into aligned rows.  The copy lives in
+// stream-ordered memory of the context's pool (safe for any streams and threads).
+b200_status RunTcgen05Aligned(b200_context* ctx, cudaStream_t stream, const b200_gemm_params* p, const b200_epilogue* epi) {
+  b200_gemm_params q = *p;
+  void* scratch[2] = {nullptr, nullptr};
+  b200_status s = B200_OK;
+  for (int i = 0; i < 2 && s == B200_OK; ++i) {
+    b200_operand& x = i == 0 ? q.a : q.b;
+    if (TmaReadable(x, p->batch)) continue;
+    const bool rows_are_k = i == 0 ? x.transpose != 0 : x.transpose == 0;
+    const int64_t outer = i == 0 ? p->m : p->n, rows = rows_are_k ? p->k : outer, cols = rows_are_k ? outer : p->k;
+    const int64_t ld = CeilDiv(cols, 8) * 8, batches = p->batch > 1 && x.batch_stride != 0 ? p->batch : 1;
+    cudaError_t e = cudaMallocFromPoolAsync(&scratch[i], static_cast<size_t>(rows) * ld * batches * 2, ctx->pool, stream);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      scratch[i] = nullptr;
+      s = Fail(B200_RESOURCE_EXHAUSTED, "b200_gemm: memory for an aligned copy of an operand: %s", cudaGetErrorString(e));
+      break;
+    }
+    s = AlignRows(ctx, stream, x, rows, cols, batches, scratch[i], ld);
+    x.ptr = scratch[i];
+    x.ld = ld;
+    x.batch_stride = batches > 1 ? rows * ld : 0;
+  }
+  if (s == B200_OK) s = RunTcgen05(ctx, stream, &q, epi);
+  for (void* d : scratch)
+    if (d != nullptr) cudaFreeAsync(d, stream);
+  return s;
+}
+
+// Worth an aligned copy: the SIMT kernel runs at about 20 TFLOP/s, the copies cost a few microseconds each.
+bool WorthAligning(const b200_gemm_params* p, const b200_epilogue* epi) {
+  b200_gemm_params q = *p;
+  for (b200_operand* x : {&q.a, &q.b})
+    if (!TmaReadable(*x, p->batch)) x->ptr = nullptr, x->ld = 8, x->batch_stride = 0;
+  return Tcgen05Supports(&q, epi) && static_cast<double>(p->m) * p->n * p->k * p->batch >= 67108864.0;
+}
+
 b200_status Validate(const b200_gemm_params* p, const b200_epilogue* epi) {
   if (p == nullptr) return Fail(B200_INVALID_ARGUMENT, "b200_gemm: null params");
   if (epi != nullptr && (epi->act < 0 || epi->act > 3))
@@ -195,7 +276,7 @@ int Route(const b200_gemm_params* p, const b200_epilogue* epi, int forced) {
   if (forced == B200_ROUTE_TCGEN05 && tc) return B200_ROUTE_TCGEN05;
   // measured on 4096 x 4096 weights: 9 vs 13 us at 1 row, 12 vs 14 at 8, 20 vs 13 at 16, 33 vs 16 at 32
   if (few && (std::min(p->m, p->n) <= 8 || !tc)) return B200_ROUTE_FEWROW;
-  if (tc) return B200_ROUTE_TCGEN05;
+  if (tc || WorthAligning(p, epi)) return B200_ROUTE_TCGEN05;
   return B200_ROUTE_SIMT;
 }
 
@@ -228,7 +309,11 @@ b200_status b200_gemm(b200_context* ctx, b200_stream stream, const b200_gemm_par
   if (epi == nullptr) epi = &none;
   const int route = Route(p, epi, ctx->force_route.load());
   if (route == B200_ROUTE_NONE) return B200_OK;
-  if (route == B200_ROUTE_TCGEN05) return RunTcgen05(ctx, stream, p, epi);
+  if (route == B200_ROUTE_TCGEN05) {
+    if (Tcgen05Supports(p, epi)) return RunTcgen05(ctx, stream, p, epi);
+    s = RunTcgen05Aligned(ctx, stream, p, epi);
+    if (s != B200_RESOURCE_EXHAUSTED) return s;   // without memory for the copies: the SIMT kernel
+  }
   if (route == B200_ROUTE_FEWROW) {
     bool vb = false;
     FewRowSupports(p, &vb);

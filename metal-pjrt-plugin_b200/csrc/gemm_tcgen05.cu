@@ -1,27 +1,38 @@
 // Dense 16-bit GEMM on the 5th-generation tensor cores:
-//   D = act(alpha * op(A) op(B) + beta * D + bias[col]),  aux = pre-activation,
+//   D[b] = act(alpha * op(A[b]) op(B[b]) + beta * D[b] + bias[col]),  aux = pre-activation,
 // the semantics of the reference's steel GEMM (metal_pjrt/blas/steel_gemm.cc:163-255,
 // kernels/steel_gemm.metal:217-225) with f32 accumulation and one rounding.
 //
-// Structure (one persistent CTA per SM, 192 threads):
-//   warp 0    TMA producer: per K step one 128 x 64 tile of op(A) and one 64 x BN tile
+// Structure (one persistent CTA per SM, 320 threads):
+//   warp 0    TMA producer: per K step one 128 x 64 tile of op(A) and one 64-deep tile
 //             of op(B), as 128-byte-swizzled boxes of cp.async.bulk.tensor (no cluster
-//             multicast), into a 4- to 8-deep shared-memory ring guarded by mbarriers;
-//   warp 1    allocates tensor memory and issues tcgen05.mma (cta_group::1, kind::f16,
-//             M = 128, N = BN, K = 16) from shared-memory descriptors; tcgen05.commit
-//             releases ring slots and signals a finished accumulator;
-//   warps 2-5 epilogue: tcgen05.ld of their 32 accumulator lanes, the fused epilogue in
-//             f32, one rounding, 64-byte row segments stored straight to D.
+//             multicast), into a shared-memory ring of up to 24 stages guarded by mbarriers;
+//   warp 1    allocates tensor memory and issues tcgen05.mma (kind::f16, K = 16) from
+//             shared-memory descriptors; tcgen05.commit releases ring slots and signals a
+//             finished accumulator;
+//   warps 2-9 epilogue: tcgen05.ld of their 32 accumulator lanes, the fused epilogue in
+//             f32, one rounding, rows gathered in shared memory and stored 128 bytes at a time.
 // Two accumulators (2 x BN of the 512 TMEM columns) let the epilogue of one tile overlap
 // the MMAs of the next.  Every wait is bounded; a wait that gives up reports
 // B200_TIMEOUT through the context's status word and the CTA unwinds (frees TMEM, returns).
 //
+// The single-thread roles are taken by an elected lane (elect.sync), not by "lane == 0": only then
+// does the compiler know that one thread runs the code and keep descriptors and addresses in
+// uniform registers.  Measured, 148 CTAs: a tcgen05.mma of 128 x 256 x 16 issued by lane 0 costs
+// 142 cycles or more whatever its N, by an elected lane 127 (N = 256), 64 (128), 48 (64).
+//
+// CG = 2: the CTAs of a pair share one 256 x 256 tile (cta_group::2, issued by the even CTA): each
+// loads its own 128 rows of A and half of B's columns, so an SM takes in 32 KB per K step instead
+// of 48 (the single-CTA form is bound by that: about 46 B per cycle and SM).
+//
 // Either operand may be transposed: a K-contiguous operand is loaded as [rows][64 k] boxes
 // (K-major descriptor), an M- or N-contiguous one as [64 k][64 rows] boxes (MN-major
-// descriptor), so nothing is transposed in memory.
+// descriptor), so nothing is transposed in memory.  Batches are the third dimension of the maps.
 #include <cooperative_groups.h>
 #include <cuda.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -33,52 +44,97 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 64;          // one 128-byte swizzle row of 16-bit elements
-constexpr int kThreads = 192;
-constexpr int kEpilogueWarps = 4;
+constexpr int kEpilogueWarps = 8;   // two per 32 TMEM lanes, half of the columns each
+constexpr int kThreads = 64 + 32 * kEpilogueWarps;
+constexpr int kMaxStages = 24;
+constexpr int kRowGroup = 8;    // tiles are walked in bands of this many row tiles, so that a wave reuses A and B in L2
+constexpr int kStagePitch = 128;                        // bytes of a staged output row; its 16-byte pieces are swizzled by row
+constexpr int kStagingBytes = kEpilogueWarps * 32 * kStagePitch;
 
 struct TcArgs {
   void* d;
   const void* bias;
   void* aux;
   int m, n, k;
-  int64_t ldd;
+  int64_t ldd, sd;       // row pitch and batch stride of D and aux
   float alpha, beta;
   int act;
-  int out_dtype;   // b200_dtype of D
   int ta, tb;
-  int tiles_m, tiles_n;
-  int split;       // CTAs of a cluster along K (grid.y); 1: persistent CTAs, no cluster
+  int tiles_m, tiles_n, batch;
+  int stages, stage_bytes;
+  int a_rows;            // rows of A in a stage: 128, or all of a smaller m (the MMA reads 128 all the same, but what the
+                         // other accumulator rows hold is never stored): a few-row product streams B through a deeper ring
+  int bcast_a, bcast_b;  // the operand is the same for every batch
+  int split;             // CTAs of a cluster along K (grid.y); 1: persistent CTAs, no cluster
   int* status;
 };
 
 // ---- PTX wrappers --------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
+// One lane of the (converged) warp, known as such to the compiler.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
+// `bar` is a shared::cluster address: with CG = 2 the barrier of the pair's even CTA.
+template <int CG>
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  if (CG == 2)
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+template <int CG>
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (CG == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
 }
+template <int CG>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+template <int CG>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
+// Arrives on `bar` once the MMAs issued so far have completed; CG = 2: on that barrier in both CTAs of the pair.
+template <int CG>
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+  if (CG == 2)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+        "h"(static_cast<uint16_t>(3))
+        : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // 32 lanes x 32 consecutive columns: thread i of the warp gets lane (base + i), columns c .. c+31
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&v)[32]) {
@@ -110,65 +166,108 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_b
 
 // Instruction descriptor for kind::f16: f32 accumulate, A/B format (0 f16, 1 bf16),
 // major-ness (0 K-major, 1 MN-major), N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t make_idesc(int ab_format, int a_mn_major, int b_mn_major, int n) {
+__host__ __device__ constexpr uint32_t make_idesc(int ab_format, int a_mn_major, int b_mn_major, int n, int m) {
   return (1u << 4) | (static_cast<uint32_t>(ab_format) << 7) | (static_cast<uint32_t>(ab_format) << 10) |
          (static_cast<uint32_t>(a_mn_major) << 15) | (static_cast<uint32_t>(b_mn_major) << 16) |
-         (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+         (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-template <int BN>
+template <int BN, int CG>
 struct Smem {
+  static constexpr int kBCols = BN / CG;             // columns of B in one CTA's shared memory
   static constexpr int kABytes = BM * BK * 2;        // 16 KB
-  static constexpr int kBBytes = BN * BK * 2;        // 32 KB at BN = 256
-  static constexpr int kStageBytes = kABytes + kBBytes;
-  // ~192 KB of ring whatever the tile width: narrow tiles stream B and need the depth
-  static constexpr int kStages = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
-  static constexpr int kTotal = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */;
+  static constexpr int kBBytes = kBCols * BK * 2;
+  static constexpr int kRing = 192 * 1024;           // cut into as many stages as fit (TcArgs::stages)
+  static constexpr int kTotal = kRing + kStagingBytes + 1024 /* alignment slack */ + 512 /* barriers */;
+  static_assert(kTotal <= 232448, "shared memory of one CTA");
 };
 
 template <typename TOut>
-__device__ __forceinline__ void epilogue_row(const TcArgs& a, const uint32_t (&v)[32], int row, int col0) {
-  TOut* D = static_cast<TOut*>(a.d);
-  TOut* AUX = static_cast<TOut*>(a.aux);
-  const TOut* bias = static_cast<const TOut*>(a.bias);
-  const int64_t o = static_cast<int64_t>(row) * a.ldd + col0;
-  const bool full = col0 + 32 <= a.n;
-  constexpr int kVec = 16 / sizeof(TOut);
-  const bool vec = full && (a.ldd % kVec == 0) && ((reinterpret_cast<uintptr_t>(D) & 15) == 0) &&
-                   (AUX == nullptr || (reinterpret_cast<uintptr_t>(AUX) & 15) == 0);
-  float x[32];
+struct alignas(16) Vec16 {
+  TOut e[16 / sizeof(TOut)];
+};
+
+template <typename TOut, int N>
+__device__ __forceinline__ void activate(int act, float (&x)[N]) {
+  if (sizeof(TOut) == 2) {
+    apply_act_16bit<N>(act, x);
+  } else if (act != 0) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    x[j] = a.alpha * __uint_as_float(v[j]);
-    if (a.beta != 0.0f && col0 + j < a.n) x[j] += a.beta * load_as_f32<TOut>(D + o + j);
-    if (bias != nullptr && col0 + j < a.n) x[j] += load_as_f32<TOut>(bias + col0 + j);
+    for (int i = 0; i < N; ++i) x[i] = apply_act(act, x[i]);
   }
-  if (vec) {
-    if (AUX != nullptr) {
+}
+
+// What is added to alpha * acc for 32 consecutive columns of one row (beta * D and the bias): read before the
+// accumulator, so that the two latencies overlap.
+template <typename TOut>
+__device__ __forceinline__ void addends(const TcArgs& a, const TOut* drow, int col0, float (&x)[32]) {
+  const TOut* bias = static_cast<const TOut*>(a.bias);
+  constexpr int kVec = 16 / sizeof(TOut);
+  const bool full = col0 + 32 <= a.n;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) x[j] = 0.0f;
+  if (a.beta != 0.0f && drow != nullptr) {
+    if (full && (reinterpret_cast<uintptr_t>(drow + col0) & 15) == 0) {
 #pragma unroll
       for (int j = 0; j < 32; j += kVec) {
-        uint4 raw;
-        TOut* e = reinterpret_cast<TOut*>(&raw);
+        const Vec16<TOut> w = *reinterpret_cast<const Vec16<TOut>*>(drow + col0 + j);
 #pragma unroll
-        for (int i = 0; i < kVec; ++i) e[i] = store_from_f32<TOut>(x[j + i]);
-        *reinterpret_cast<uint4*>(AUX + o + j) = raw;
+        for (int i = 0; i < kVec; ++i) x[j + i] = a.beta * load_as_f32<TOut>(&w.e[i]);
       }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (col0 + j < a.n) x[j] = a.beta * load_as_f32<TOut>(drow + col0 + j);
     }
+  }
+  if (bias != nullptr) {
+    if (full && (reinterpret_cast<uintptr_t>(bias + col0) & 15) == 0) {
 #pragma unroll
-    for (int j = 0; j < 32; j += kVec) {
-      uint4 raw;
-      TOut* e = reinterpret_cast<TOut*>(&raw);
+      for (int j = 0; j < 32; j += kVec) {
+        const Vec16<TOut> w = *reinterpret_cast<const Vec16<TOut>*>(bias + col0 + j);
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) e[i] = store_from_f32<TOut>(apply_act(a.act, x[j + i]));
-      *reinterpret_cast<uint4*>(D + o + j) = raw;
+        for (int i = 0; i < kVec; ++i) x[j + i] += load_as_f32<TOut>(&w.e[i]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (col0 + j < a.n) x[j] += load_as_f32<TOut>(bias + col0 + j);
+    }
+  }
+}
+
+// Where byte b of staged row r lies: 16-byte accesses down a column of rows hit different banks.
+__device__ __forceinline__ int staged(int r, int b) { return r * kStagePitch + ((((b >> 4) ^ r) & 7) << 4) + (b & 15); }
+
+// 32 staged rows of 128 bytes -> global, a row (or four rows by 16-byte pieces) per instruction.
+template <typename TOut>
+__device__ __forceinline__ void store_rows(const uint8_t* st, TOut* out, int64_t ld, int row0, int rows, int col0, int cols, int lane) {
+  constexpr int kCols = 128 / sizeof(TOut);
+  constexpr int kVec = 16 / sizeof(TOut);
+  const uintptr_t base = reinterpret_cast<uintptr_t>(out);
+  if (cols >= kCols && base % 16 == 0 && ld % kVec == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = 4 * i + (lane >> 3);
+      if (r < rows)
+        *reinterpret_cast<uint4*>(out + static_cast<int64_t>(row0 + r) * ld + col0 + (lane & 7) * kVec) =
+            *reinterpret_cast<const uint4*>(st + staged(r, (lane & 7) * 16));
+    }
+  } else if (sizeof(TOut) == 2 && base % 4 == 0 && ld % 2 == 0) {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+      TOut* o = out + static_cast<int64_t>(row0 + r) * ld + col0 + 2 * lane;
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(st + staged(r, 4 * lane));
+      if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(o) = w;
+      else if (2 * lane < cols) *o = *reinterpret_cast<const TOut*>(&w);
     }
   } else {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+      TOut* o = out + static_cast<int64_t>(row0 + r) * ld + col0;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if (col0 + j < a.n) {
-        if (AUX != nullptr) AUX[o + j] = store_from_f32<TOut>(x[j]);
-        D[o + j] = store_from_f32<TOut>(apply_act(a.act, x[j]));
-      }
+      for (int c = 0; c < kCols; c += 32)
+        if (c + lane < cols) o[c + lane] = *reinterpret_cast<const TOut*>(st + staged(r, (c + lane) * static_cast<int>(sizeof(TOut))));
     }
   }
 }
@@ -176,9 +275,7 @@ __device__ __forceinline__ void epilogue_row(const TcArgs& a, const uint32_t (&v
 // The same epilogue for 4 consecutive columns (the split-K reduction, where a warp owns a
 // row and its lanes adjacent float4s, so that the reads of the peers' tiles coalesce).
 template <typename TOut>
-__device__ __forceinline__ void epilogue_quad(const TcArgs& a, const float (&acc)[4], int row, int col0) {
-  TOut* D = static_cast<TOut*>(a.d);
-  TOut* AUX = static_cast<TOut*>(a.aux);
+__device__ __forceinline__ void epilogue_quad(const TcArgs& a, const float (&acc)[4], TOut* D, TOut* AUX, int row, int col0) {
   const TOut* bias = static_cast<const TOut*>(a.bias);
   const int64_t o = static_cast<int64_t>(row) * a.ldd + col0;
   float x[4];
@@ -190,6 +287,8 @@ __device__ __forceinline__ void epilogue_quad(const TcArgs& a, const float (&acc
       if (bias != nullptr) x[j] += load_as_f32<TOut>(bias + col0 + j);
     }
   }
+  float y[4] = {x[0], x[1], x[2], x[3]};
+  activate<TOut>(a.act, y);
   constexpr size_t kBytes = 4 * sizeof(TOut);
   const bool vec = col0 + 4 <= a.n && (a.ldd % 4 == 0) && (reinterpret_cast<uintptr_t>(D) % kBytes == 0) &&
                    (AUX == nullptr || reinterpret_cast<uintptr_t>(AUX) % kBytes == 0);
@@ -199,7 +298,7 @@ __device__ __forceinline__ void epilogue_quad(const TcArgs& a, const float (&acc
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       pa.e[j] = store_from_f32<TOut>(x[j]);
-      pd.e[j] = store_from_f32<TOut>(apply_act(a.act, x[j]));
+      pd.e[j] = store_from_f32<TOut>(y[j]);
     }
     if (AUX != nullptr) *reinterpret_cast<Pack*>(AUX + o) = pa;
     *reinterpret_cast<Pack*>(D + o) = pd;
@@ -208,50 +307,86 @@ __device__ __forceinline__ void epilogue_quad(const TcArgs& a, const float (&acc
     for (int j = 0; j < 4; ++j) {
       if (col0 + j < a.n) {
         if (AUX != nullptr) AUX[o + j] = store_from_f32<TOut>(x[j]);
-        D[o + j] = store_from_f32<TOut>(apply_act(a.act, x[j]));
+        D[o + j] = store_from_f32<TOut>(y[j]);
       }
     }
   }
 }
 
-template <int BN, typename TOut>
+// One arrival on barrier `bar` of CTA `rank`, without ordering this thread's global stores before it (a release
+// at cluster scope would wait for them): tcgen05.wait::ld and the tcgen05 fence order what matters here.
+__device__ __forceinline__ void mbar_arrive_relaxed(uint64_t* bar, uint32_t rank) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(smem_u32(bar)),
+      "r"(rank)
+      : "memory");
+}
+
+struct TileAt {
+  int b, tm, tn;
+};
+__device__ __forceinline__ TileAt tile_at(const TcArgs& a, int tile) {
+  const int per = a.tiles_m * a.tiles_n;
+  TileAt t;
+  t.b = tile / per;
+  const int r = tile - t.b * per;
+  const int band = r / (kRowGroup * a.tiles_n), in = r - band * kRowGroup * a.tiles_n;
+  const int rows = min(kRowGroup, a.tiles_m - band * kRowGroup);
+  t.tm = band * kRowGroup + in % rows;
+  t.tn = in / rows;
+  return t;
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(p)), "r"(rank));
+  return ra;
+}
+
+template <int BN, int CG, typename TOut>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                    const uint32_t idesc) {
-  using S = Smem<BN>;
-  constexpr int kStages = S::kStages;
+  using S = Smem<BN, CG>;
+  const int stages = a.stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * S::kStageBytes);
-  uint64_t* empty = full + kStages;
-  uint64_t* tfull = empty + kStages;
+  uint8_t* staging = smem + S::kRing;
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + kStagingBytes);
+  uint64_t* empty = full + kMaxStages;
+  uint64_t* tfull = empty + kMaxStages;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int num_tiles = a.tiles_m * a.tiles_n;
+  const int num_tiles = a.tiles_m * a.tiles_n * a.batch;
   const int k_iters = (a.k + BK - 1) / BK;
+  const int rank = CG == 2 ? static_cast<int>(blockIdx.x & 1) : 0;   // CTA of the pair
+  const int tile0 = static_cast<int>(blockIdx.x) / CG, tile_step = static_cast<int>(gridDim.x) / CG;
+  const bool solo = CG == 2 || a.split == 1;
   // With K split across a cluster, grid.x is the tile count (one tile per CTA) and CTA
   // blockIdx.y accumulates k steps [ki_begin, ki_end) of it.
-  const int ki_begin = a.split > 1 ? static_cast<int>(blockIdx.y) * k_iters / a.split : 0;
-  const int ki_end = a.split > 1 ? (static_cast<int>(blockIdx.y) + 1) * k_iters / a.split : k_iters;
+  const int ki_begin = solo ? 0 : static_cast<int>(blockIdx.y) * k_iters / a.split;
+  const int ki_end = solo ? k_iters : (static_cast<int>(blockIdx.y) + 1) * k_iters / a.split;
   constexpr int kPartLd = BN + 4;          // row pitch (floats) of the partial tile in shared memory
   constexpr uint32_t kTmemCols = 2 * BN;   // two accumulators; a power of two >= 32
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
-      mbar_init(&tempty[i], kEpilogueWarps);
+      mbar_init(&tempty[i], CG * kEpilogueWarps);
     }
     mbar_fence_init();
   }
-  if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+  if (warp == 1) tmem_alloc<CG>(tmem_slot, kTmemCols);
   tc_fence_before();
   __syncthreads();
+  if (CG == 2) cg::this_cluster().sync();   // the pair's barriers exist before anyone arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();               // A, B (and D under beta) may come from the previous kernel
@@ -259,127 +394,187 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0) {
     // ---------------- TMA producer (one lane)
-    if (lane == 0) {
-      int it = 0;
+    if (elect_one()) {
+      const uint32_t a_bytes = static_cast<uint32_t>(a.a_rows) * BK * 2;
+      int s = 0;
+      uint32_t parity = 1;   // the first lap waits for nothing
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int tm = tile % a.tiles_m, tn = tile / a.tiles_m;
-        for (int ki = ki_begin; ki < ki_end && ok; ++ki, ++it) {
-          const int s = it % kStages, use = it / kStages;
-          if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1)) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+        const TileAt t = tile_at(a, tile);
+        const int row0 = (t.tm * CG + rank) * BM, col0 = t.tn * BN + rank * S::kBCols;
+        const int ba = a.bcast_a ? 0 : t.b, bb = a.bcast_b ? 0 : t.b;
+        for (int ki = ki_begin; ki < ki_end; ++ki) {
+          if (!mbar_wait_bounded(&empty[s], parity)) {
             report_timeout(a.status, 300 + s);
             ok = false;
             break;
           }
-          uint8_t* As = smem + s * S::kStageBytes;
-          uint8_t* Bs = As + S::kABytes;
-          mbar_expect_tx(&full[s], S::kStageBytes);
+          const uint32_t As = smem_u32(smem + s * a.stage_bytes), Bs = As + a_bytes;
+          const uint32_t bar = CG == 2 ? cluster_addr(&full[s], 0) : smem_u32(&full[s]);
+          if (rank == 0) mbar_expect_tx(&full[s], CG * a.stage_bytes);
           if (!a.ta) {
-            tma_load_2d(As, &tmA, ki * BK, tm * BM, &full[s]);                 // [128 m][64 k]
+            tma_load_3d<CG>(As, &tmA, ki * BK, row0, ba, bar);                   // [128 m][64 k]
           } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j)                                    // [64 k][64 m] boxes
-              tma_load_2d(As + j * 8192, &tmA, tm * BM + j * 64, ki * BK, &full[s]);
+            for (int j = 0; j < BM / 64; ++j)                                      // [64 k][64 m] boxes
+              tma_load_3d<CG>(As + j * 8192, &tmA, row0 + j * 64, ki * BK, ba, bar);
           }
           if (a.tb) {
-            tma_load_2d(Bs, &tmB, ki * BK, tn * BN, &full[s]);                 // [BN n][64 k]
+            tma_load_3d<CG>(Bs, &tmB, ki * BK, col0, bb, bar);                   // [n][64 k]
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j)                                    // [64 k][64 n] boxes
-              tma_load_2d(Bs + j * 8192, &tmB, tn * BN + j * 64, ki * BK, &full[s]);
+            for (int j = 0; j < S::kBCols / 64; ++j)                               // [64 k][64 n] boxes
+              tma_load_3d<CG>(Bs + j * 8192, &tmB, col0 + j * 64, ki * BK, bb, bar);
           }
+          if (++s == stages) s = 0, parity ^= 1;
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    // ---------------- MMA issuer (one lane)
-    if (lane == 0) {
-      int it = 0, tcount = 0;
+    // ---------------- MMA issuer (one lane; of a pair, the even CTA's)
+    if (rank == 0 && elect_one()) {
+      int s = 0, tcount = 0;
+      uint32_t parity = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
-        const int acc = tcount & 1, use_acc = tcount >> 1;
-        if (use_acc > 0 && !mbar_wait_bounded(&tempty[acc], (use_acc - 1) & 1)) {
+      const uint64_t desc_a0 = a.ta ? make_desc(smem_u32(smem), 8192, 1024) : make_desc(smem_u32(smem), 16, 1024);
+      const uint32_t b0 = smem_u32(smem) + static_cast<uint32_t>(a.a_rows) * BK * 2;
+      const uint64_t desc_b0 = a.tb ? make_desc(b0, 16, 1024) : make_desc(b0, 8192, 1024);
+      const uint64_t step_a = a.ta ? 2048 >> 4 : 32 >> 4, step_b = a.tb ? 32 >> 4 : 2048 >> 4;   // 16 k further
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step, ++tcount) {
+        const int acc = tcount & 1;
+        if (!mbar_wait_bounded(&tempty[acc], ((tcount >> 1) & 1) ^ 1)) {
           report_timeout(a.status, 310 + acc);
           ok = false;
           break;
         }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
-        for (int ki = ki_begin; ki < ki_end && ok; ++ki, ++it) {
-          const int s = it % kStages;
-          if (!mbar_wait_bounded(&full[s], (it / kStages) & 1)) {
+        for (int ki = ki_begin; ki < ki_end; ++ki) {
+          if (!mbar_wait_bounded(&full[s], parity)) {
             report_timeout(a.status, 320 + s);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * S::kStageBytes);
-          const uint32_t b_addr = a_addr + S::kABytes;
+          uint64_t da = desc_a0 + static_cast<uint64_t>(s * (a.stage_bytes >> 4));
+          uint64_t db = desc_b0 + static_cast<uint64_t>(s * (a.stage_bytes >> 4));
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = a.ta ? make_desc(a_addr + kk * 2048, 8192, 1024) : make_desc(a_addr + kk * 32, 16, 1024);
-            const uint64_t db = a.tb ? make_desc(b_addr + kk * 32, 16, 1024) : make_desc(b_addr + kk * 2048, 8192, 1024);
-            umma_f16(tmem_d, da, db, idesc, (ki > ki_begin || kk > 0) ? 1u : 0u);
+            umma_f16<CG>(tmem_d, da, db, idesc, (ki > ki_begin || kk > 0) ? 1u : 0u);
+            da += step_a;
+            db += step_b;
           }
-          umma_commit(&empty[s]);     // the slot is free once these MMAs have read it
+          umma_commit<CG>(&empty[s]);     // the slot is free once these MMAs have read it
+          if (++s == stages) s = 0, parity ^= 1;
         }
-        if (ok) umma_commit(&tfull[acc]);
+        if (ok) umma_commit<CG>(&tfull[acc]);
       }
     }
+    __syncwarp();
   } else {
-    // ---------------- epilogue warps: TMEM lanes 32 q .. 32 q + 31
+    // ---------------- epilogue warps: TMEM lanes 32 q .. 32 q + 31, columns c_lo .. c_lo + BN / 2 - 1
     const int q = warp & 3;
+    const int c_lo = ((warp - 2) >> 2) * (BN / 2);
+    uint8_t* st = staging + (warp - 2) * 32 * kStagePitch;
+    constexpr int kCols = 128 / static_cast<int>(sizeof(TOut));   // columns gathered per store pass
+    constexpr int kPass = kCols < BN / 2 ? kCols : BN / 2;
+    constexpr int kVec = 16 / static_cast<int>(sizeof(TOut));
+    auto accumulator_free = [&](int acc) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_relaxed(&tempty[acc], 0);
+        else mbar_arrive(&tempty[acc]);
+      }
+    };
     int tcount = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
-      const int tm = tile % a.tiles_m, tn = tile / a.tiles_m;
+    for (int tile = tile0; tile < num_tiles; tile += tile_step, ++tcount) {
+      const TileAt t = tile_at(a, tile);
       const int acc = tcount & 1;
       if (!mbar_wait_bounded(&tfull[acc], (tcount >> 1) & 1)) {
         report_timeout(a.status, 330 + acc);
-        ok = false;
         break;
       }
       tc_fence_after();
-      const int row = tm * BM + 32 * q + lane;
+      bool drained = false;
+      const uint32_t tmem_row = tmem_base + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(acc * BN);
+      if (!solo) {
+        // this CTA's K slice only: park the f32 partial in the (now idle) ring
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(acc * BN + c0), v);
-        const int col0 = tn * BN + c0;
-        if (a.split > 1) {
-          // this CTA's K slice only: park the f32 partial in the (now idle) ring
+        for (int c0 = c_lo; c0 < c_lo + BN / 2; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld_32x32(tmem_row + static_cast<uint32_t>(c0), v);
           float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem) + (32 * q + lane) * kPartLd + c0);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             dst[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
                                  __uint_as_float(v[4 * j + 3]));
-        } else if (row < a.m && col0 < a.n) {
-          epilogue_row<TOut>(a, v, row, col0);
+        }
+      } else {
+        const int row0 = (t.tm * CG + rank) * BM + 32 * q, rows = min(32, a.m - row0);
+        TOut* D = static_cast<TOut*>(a.d) + t.b * a.sd;
+        TOut* AUX = a.aux != nullptr ? static_cast<TOut*>(a.aux) + t.b * a.sd : nullptr;
+        const TOut* drow = lane < rows ? D + static_cast<int64_t>(row0 + lane) * a.ldd : nullptr;
+        if (rows > 0) {
+#pragma unroll 1
+          for (int c0 = c_lo; c0 < c_lo + BN / 2 && t.tn * BN + c0 < a.n; c0 += kPass) {
+            const int col0 = t.tn * BN + c0;
+#pragma unroll 1
+            for (int pass = AUX != nullptr ? 0 : 1; pass < 2; ++pass) {   // 0: the pre-activation to aux, 1: D
+#pragma unroll
+              for (int h = 0; h < kPass; h += 32) {
+                uint32_t v[32];
+                float x[32];
+                addends<TOut>(a, drow, col0 + h, x);
+                tmem_ld_32x32(tmem_row + static_cast<uint32_t>(c0 + h), v);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) x[j] = fmaf(a.alpha, __uint_as_float(v[j]), x[j]);
+                if (pass == 1) activate<TOut>(a.act, x);
+#pragma unroll
+                for (int j = 0; j < 32; j += kVec) {
+                  Vec16<TOut> w;
+#pragma unroll
+                  for (int i = 0; i < kVec; ++i) w.e[i] = store_from_f32<TOut>(x[j + i]);
+                  *reinterpret_cast<Vec16<TOut>*>(st + staged(lane, (h + j) * static_cast<int>(sizeof(TOut)))) = w;
+                }
+              }
+              __syncwarp();
+              if (pass == 1 && (c0 + kPass >= c_lo + BN / 2 || col0 + kPass >= a.n)) {   // the last read of this accumulator
+                accumulator_free(acc);
+                drained = true;
+              }
+              store_rows<TOut>(st, pass == 0 ? AUX : D, a.ldd, row0, rows, col0, min(kPass, a.n - col0), lane);
+              __syncwarp();
+            }
+          }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
+      if (!drained) accumulator_free(acc);
     }
   }
-  if (a.split > 1) {
-    // K split: every CTA of the cluster finishes rows [rank, rank + 1) * 128 / split of the
+  if (CG == 2) {
+    cg::this_cluster().sync();   // the pair's barriers and tensor memory are in use until both are done
+  } else if (a.split > 1) {
+    // K split: every CTA of the cluster finishes its share of the rows of the
     // tile from all the partial tiles, read through distributed shared memory.
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     if (warp >= 2) {
-      const int tile = blockIdx.x, tm = tile % a.tiles_m, tn = tile / a.tiles_m;
-      const int rows_per_rank = BM / a.split;
+      const TileAt t = tile_at(a, blockIdx.x);
+      TOut* D = static_cast<TOut*>(a.d) + t.b * a.sd;
+      TOut* AUX = a.aux != nullptr ? static_cast<TOut*>(a.aux) + t.b * a.sd : nullptr;
+      const int tile_rows = min(BM, a.m - t.tm * BM), rows_per_rank = (tile_rows + a.split - 1) / a.split;
       const float* part = reinterpret_cast<const float*>(smem);
       // a warp per row, lanes on adjacent float4s: 512-byte runs of every peer's tile
       for (int rr = warp - 2; rr < rows_per_rank; rr += kEpilogueWarps) {
         const int r = static_cast<int>(blockIdx.y) * rows_per_rank + rr;
-        const int row = tm * BM + r;
-        if (row >= a.m) break;
+        const int row = t.tm * BM + r;
+        if (r >= tile_rows) break;
 #pragma unroll
-        for (int t = 0; t < BN / 128 + (BN < 128 ? 1 : 0); ++t) {
-          const int c = t * 128 + 4 * lane;
-          if (c >= BN || tn * BN + c >= a.n) continue;
+        for (int u = 0; u < BN / 128 + (BN < 128 ? 1 : 0); ++u) {
+          const int c = u * 128 + 4 * lane;
+          if (c >= BN || t.tn * BN + c >= a.n) continue;
           float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
           float4 v[8];
 #pragma unroll
@@ -394,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             sum[2] += v[peer].z;
             sum[3] += v[peer].w;
           }
-          epilogue_quad<TOut>(a, sum, row, tn * BN + c);
+          epilogue_quad<TOut>(a, sum, D, AUX, row, t.tn * BN + c);
         }
       }
     }
@@ -404,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc<CG>(tmem_base, kTmemCols);
   }
 }
 
@@ -429,56 +624,64 @@ EncodeTiledFn Encoder() {
   return fn;
 }
 
-// A 2-D map over a row-major matrix: `inner` contiguous elements per row, `outer`
-// rows `ld` elements apart; boxes of box_inner x box_outer, 128-byte swizzle.
-bool MakeMap(CUtensorMap* map, int dtype, const void* base, int64_t inner, int64_t outer, int64_t ld, int box_inner,
-             int box_outer) {
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer)};
-  const cuuint32_t estr[2] = {1, 1};
+// A 3-D map over `batch` row-major matrices: `inner` contiguous elements per row, `outer`
+// rows `ld` elements apart; boxes of box_inner x box_outer x 1, 128-byte swizzle.
+bool MakeMap(CUtensorMap* map, int dtype, const void* base, int64_t inner, int64_t outer, int64_t ld, int64_t batch,
+             int64_t batch_stride, int box_inner, int box_outer) {
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(inner), static_cast<cuuint64_t>(outer), static_cast<cuuint64_t>(batch)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(batch > 1 ? batch_stride : ld * outer) * 2};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer), 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = Encoder()(map, dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                               2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
-template <int BN, typename TOut>
+template <int BN, int CG, typename TOut>
 cudaError_t LaunchTc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, uint32_t idesc, int grid,
                      cudaStream_t stream) {
-  static_assert(BM * (BN + 4) * 4 <= Smem<BN>::kStages * Smem<BN>::kStageBytes, "partial tile must fit the ring");
-  auto kernel = gemm_tc_kernel<BN, TOut>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<BN>::kTotal);
+  static_assert(BM * (BN / CG + 4) * 4 <= Smem<BN, CG>::kRing, "partial tile must fit the ring");
+  auto kernel = gemm_tc_kernel<BN, CG, TOut>;
+  static std::atomic<uint64_t> ready{0};   // per device: the shared-memory limit is raised
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
+  if ((ready.load(std::memory_order_relaxed) >> (dev & 63) & 1) == 0) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<BN, CG>::kTotal);
+    if (e != cudaSuccess) return e;
+    ready.fetch_or(1ull << (dev & 63));
+  }
   LaunchCfg lc;
-  lc.grid = dim3(grid, a.split, 1);
+  lc.grid = dim3(CG * grid, a.split, 1);
   lc.block = dim3(kThreads);
-  lc.smem = Smem<BN>::kTotal;
+  lc.smem = Smem<BN, CG>::kTotal;
   lc.stream = stream;
   lc.pdl = true;
+  lc.cluster_x = CG;
   lc.cluster_y = a.split;
   return Launch(lc, kernel, ma, mb, a, idesc);
 }
 
 // How many clusters of `split` CTAs of this kernel the device holds at once (a GPC takes
 // only whole clusters, so this can be well below SMs / split).  Cached per shape of launch.
-template <int BN, typename TOut>
+template <int BN, int CG, typename TOut>
 int ResidentClusters(int split) {
   static std::mutex mu;
   static int cached[9] = {0};
   std::lock_guard<std::mutex> lock(mu);
   if (cached[split] == 0) {
-    auto kernel = gemm_tc_kernel<BN, TOut>;
+    auto kernel = gemm_tc_kernel<BN, CG, TOut>;
     int n = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<BN>::kTotal) == cudaSuccess) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<BN, CG>::kTotal) == cudaSuccess) {
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(16, split, 1);
+      cfg.gridDim = dim3(16 * CG, split, 1);
       cfg.blockDim = dim3(kThreads);
-      cfg.dynamicSmemBytes = Smem<BN>::kTotal;
+      cfg.dynamicSmemBytes = Smem<BN, CG>::kTotal;
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = 1;
+      attr.val.clusterDim.x = CG;
       attr.val.clusterDim.y = split;
       attr.val.clusterDim.z = 1;
       cfg.attrs = &attr;
@@ -491,66 +694,91 @@ int ResidentClusters(int split) {
   return cached[split] > 0 ? cached[split] : 0;
 }
 
-template <int BN>
+template <int BN, int CG>
 int ResidentClustersFor(int out_dtype, int split) {
-  if (out_dtype == B200_F32) return ResidentClusters<BN, float>(split);
-  if (out_dtype == B200_BF16) return ResidentClusters<BN, __nv_bfloat16>(split);
-  return ResidentClusters<BN, __half>(split);
+  if (out_dtype == B200_F32) return ResidentClusters<BN, CG, float>(split);
+  if (out_dtype == B200_BF16) return ResidentClusters<BN, CG, __nv_bfloat16>(split);
+  return ResidentClusters<BN, CG, __half>(split);
+}
+
+template <int BN, int CG>
+cudaError_t LaunchFor(int out_dtype, const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, uint32_t idesc, int grid,
+                      cudaStream_t stream) {
+  if (out_dtype == B200_F32) return LaunchTc<BN, CG, float>(ma, mb, a, idesc, grid, stream);
+  if (out_dtype == B200_BF16) return LaunchTc<BN, CG, __nv_bfloat16>(ma, mb, a, idesc, grid, stream);
+  return LaunchTc<BN, CG, __half>(ma, mb, a, idesc, grid, stream);
 }
 
 }  // namespace
 
 namespace b200 {
 
+bool TmaReadable(const b200_operand& x, int64_t batch) {
+  // 16-byte aligned bases, row pitches and batch strides that are multiples of 16 bytes
+  if (!Aligned(x.ptr, 16) || x.ld % 8 != 0) return false;
+  return batch == 1 || x.batch_stride == 0 || (x.batch_stride % 8 == 0 && x.ld > 0 && x.batch_stride % x.ld == 0);
+}
+
 bool Tcgen05Supports(const b200_gemm_params* p, const b200_epilogue* epi) {
   (void)epi;
   if (p->a.dtype != B200_BF16 && p->a.dtype != B200_F16) return false;
   if (p->b.dtype != p->a.dtype) return false;
-  if (p->batch != 1 || p->k < 1) return false;
+  if (p->k < 1) return false;
   if (Encoder() == nullptr) return false;
-  // TMA: 16-byte aligned bases, row pitches that are multiples of 16 bytes
-  if (!Aligned(p->a.ptr, 16) || !Aligned(p->b.ptr, 16)) return false;
-  if (p->a.ld % 8 != 0 || p->b.ld % 8 != 0) return false;
+  if (!TmaReadable(p->a, p->batch) || !TmaReadable(p->b, p->batch)) return false;
   if (p->m > (1 << 30) || p->n > (1 << 30) || p->k > (1 << 30)) return false;
-  return true;
+  return CeilDiv(p->m, BM) * CeilDiv(p->n, 64) * p->batch <= INT32_MAX;
 }
 
 b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_params* p, const b200_epilogue* epi) {
   const int ta = p->a.transpose, tb = p->b.transpose;
-  const int64_t m = p->m, n = p->n, k = p->k;
-  // 128 x 256 tiles; narrower ones (128, 64 columns) when that is what it takes to spread
-  // a few-row problem, which only streams B, over more SMs
-  const int64_t tiles_m = CeilDiv(m, BM), k_iters = CeilDiv(k, BK);
-  // Tile width and K split by a small cost model (microseconds).  A k step of a 128 x bn
-  // tile costs what the SM's share of L2 bandwidth or the MMAs take, whichever is longer
-  // (measured: 0.55 / 0.43 / 0.375 us for bn = 256 / 128 / 64); tiles run in waves over the
-  // SMs.  When the tiles leave SMs idle, a cluster of 2/4/8 CTAs splits one tile's K loop
-  // (a serial chain on one SM otherwise) and adds the partial tiles through distributed
-  // shared memory, for a fixed cost of the cluster barriers and the extra pass.
-  int bn = 256, split = 1;
+  const int64_t m = p->m, n = p->n, k = p->k, batch = p->batch;
+  // Tile shape and K split by a small cost model (microseconds); tiles run in waves over
+  // the SMs (256 x 256 tiles over pairs of SMs).  When the tiles leave SMs idle, a cluster of
+  // 2/4/8 CTAs splits one tile's K loop (a serial chain on one SM otherwise) and adds the partial
+  // tiles through distributed shared memory, for a fixed cost of the cluster barriers and the extra pass.
+  const int64_t k_iters = CeilDiv(k, BK);
+  const int a_rows = ta ? BM : static_cast<int>(std::min<int64_t>(BM, CeilDiv(m, 8) * 8));
+  // A k step moves a_rows x 64 of A and bn x 64 of B into an SM at about 0.1 MB/us; the MMAs of a 256-wide
+  // tile take 0.27 us.  epi: tcgen05.ld, the fused epilogue and the stores of one tile, overlapped with the next tile's loop.
+  auto waves_cost = [&](int64_t tiles, int64_t slots, double t_iter, double epi) {
+    return static_cast<double>(CeilDiv(tiles, slots)) * std::max(k_iters * t_iter, epi) + epi;
+  };
+  int bn = 256, group = 1, split = 1;
   double best = 1e30;
-  for (int cand : {256, 128, 64}) {
-    const double t_iter = cand == 256 ? 0.55 : (cand == 128 ? 0.43 : 0.375);
-    const int64_t tiles = tiles_m * CeilDiv(n, cand);
-    const double whole = static_cast<double>(CeilDiv(tiles, ctx->sm_count)) * k_iters * t_iter;
-    if (whole < best) best = whole, bn = cand, split = 1;
+  {
+    const int pairs = ResidentClustersFor<256, 2>(p->c.dtype, 1);
+    const int64_t tiles = CeilDiv(m, 2 * BM) * CeilDiv(n, 256) * batch;
+    if (pairs > 0 && m > BM) best = waves_cost(tiles, pairs, 0.39, 2.5), group = 2;
+  }
+  for (int cand : {128, 64}) {
+    // 64 columns are 128-byte pieces of B's rows, which stream at about 0.8 of the rate of 256-byte ones
+    const double t_iter = (a_rows + cand) * (BK * 2) * (cand == 64 ? 1.25e-5 : 1e-5), epi = cand == 128 ? 1.3 : 0.8;
+    const int64_t tiles = CeilDiv(m, BM) * CeilDiv(n, cand) * batch;
+    const double whole = waves_cost(tiles, ctx->sm_count, t_iter, epi);
+    if (whole < best) best = whole, bn = cand, group = 1, split = 1;
     for (int sp = 2; sp <= 8; sp *= 2) {
       if (tiles * sp > ctx->sm_count || k_iters / sp < 4) break;
-      const int resident = cand == 256 ? ResidentClustersFor<256>(p->c.dtype, sp)
-                                       : (cand == 128 ? ResidentClustersFor<128>(p->c.dtype, sp) : ResidentClustersFor<64>(p->c.dtype, sp));
+      const int resident = cand == 128 ? ResidentClustersFor<128, 1>(p->c.dtype, sp) : ResidentClustersFor<64, 1>(p->c.dtype, sp);
       if (tiles > resident) continue;   // a second wave of clusters would double the time
-      const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 4.0;
-      if (cost < best) best = cost, bn = cand, split = sp;
+      const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 1.5 + epi;
+      if (cost < best) best = cost, bn = cand, group = 1, split = sp;
     }
   }
+  TcArgs a;
+  a.a_rows = a_rows;
+  a.stage_bytes = (a_rows + bn / group) * BK * 2;
+  a.stages = std::min(kMaxStages, 192 * 1024 / a.stage_bytes);
+  a.bcast_a = batch > 1 && p->a.batch_stride == 0;
+  a.bcast_b = batch > 1 && p->b.batch_stride == 0;
+  const int64_t ba = a.bcast_a ? 1 : batch, bb = a.bcast_b ? 1 : batch;
   CUtensorMap ma, mb;
   bool ok;
-  if (!ta) ok = MakeMap(&ma, p->a.dtype, p->a.ptr, k, m, p->a.ld, BK, BM);     // A [m][k]
-  else ok = MakeMap(&ma, p->a.dtype, p->a.ptr, m, k, p->a.ld, 64, BK);         // A stored [k][m]
-  if (tb) ok = ok && MakeMap(&mb, p->b.dtype, p->b.ptr, k, n, p->b.ld, BK, bn); // B stored [n][k]
-  else ok = ok && MakeMap(&mb, p->b.dtype, p->b.ptr, n, k, p->b.ld, 64, BK);   // B [k][n]
+  if (!ta) ok = MakeMap(&ma, p->a.dtype, p->a.ptr, k, m, p->a.ld, ba, p->a.batch_stride, BK, a.a_rows);           // A [m][k]
+  else ok = MakeMap(&ma, p->a.dtype, p->a.ptr, m, k, p->a.ld, ba, p->a.batch_stride, 64, BK);                     // A stored [k][m]
+  if (tb) ok = ok && MakeMap(&mb, p->b.dtype, p->b.ptr, k, n, p->b.ld, bb, p->b.batch_stride, BK, bn / group);     // B stored [n][k]
+  else ok = ok && MakeMap(&mb, p->b.dtype, p->b.ptr, n, k, p->b.ld, bb, p->b.batch_stride, 64, BK);               // B [k][n]
   if (!ok) return Stick(ctx, Fail(B200_INTERNAL, "b200_gemm: cuTensorMapEncodeTiled refused the operand layout"));
-  TcArgs a;
   a.d = p->c.ptr;
   a.bias = epi->bias;
   a.aux = epi->aux;
@@ -558,33 +786,28 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
   a.n = static_cast<int>(n);
   a.k = static_cast<int>(k);
   a.ldd = p->c.ld;
+  a.sd = batch > 1 ? p->c.batch_stride : 0;
   a.alpha = static_cast<float>(p->alpha);
   a.beta = static_cast<float>(p->beta);
   a.act = epi->act;
-  a.out_dtype = p->c.dtype;
   a.ta = ta;
   a.tb = tb;
-  a.tiles_m = static_cast<int>(tiles_m);
+  a.tiles_m = static_cast<int>(CeilDiv(m, BM * group));
   a.tiles_n = static_cast<int>(CeilDiv(n, bn));
+  a.batch = static_cast<int>(batch);
   a.split = split;
   a.status = ctx->dev_status;
-  const int64_t tiles = static_cast<int64_t>(a.tiles_m) * a.tiles_n;
-  const int grid = split > 1 ? static_cast<int>(tiles) : static_cast<int>(std::min<int64_t>(tiles, ctx->sm_count));
-  const uint32_t idesc = make_idesc(p->a.dtype == B200_BF16 ? 1 : 0, ta ? 1 : 0, tb ? 0 : 1, bn);
-  cudaError_t e;
+  const int64_t tiles = static_cast<int64_t>(a.tiles_m) * a.tiles_n * batch;
+  const uint32_t idesc = make_idesc(p->a.dtype == B200_BF16 ? 1 : 0, ta ? 1 : 0, tb ? 0 : 1, bn, BM * group);
   const int out = p->c.dtype;
-  if (bn == 256) {
-    if (out == B200_F32) e = LaunchTc<256, float>(ma, mb, a, idesc, grid, stream);
-    else if (out == B200_BF16) e = LaunchTc<256, __nv_bfloat16>(ma, mb, a, idesc, grid, stream);
-    else e = LaunchTc<256, __half>(ma, mb, a, idesc, grid, stream);
-  } else if (bn == 128) {
-    if (out == B200_F32) e = LaunchTc<128, float>(ma, mb, a, idesc, grid, stream);
-    else if (out == B200_BF16) e = LaunchTc<128, __nv_bfloat16>(ma, mb, a, idesc, grid, stream);
-    else e = LaunchTc<128, __half>(ma, mb, a, idesc, grid, stream);
+  cudaError_t e;
+  if (group == 2) {
+    const int grid = static_cast<int>(std::min<int64_t>(tiles, ResidentClustersFor<256, 2>(out, 1)));
+    e = LaunchFor<256, 2>(out, ma, mb, a, idesc, grid, stream);
   } else {
-    if (out == B200_F32) e = LaunchTc<64, float>(ma, mb, a, idesc, grid, stream);
-    else if (out == B200_BF16) e = LaunchTc<64, __nv_bfloat16>(ma, mb, a, idesc, grid, stream);
-    else e = LaunchTc<64, __half>(ma, mb, a, idesc, grid, stream);
+    const int grid = split > 1 ? static_cast<int>(tiles) : static_cast<int>(std::min<int64_t>(tiles, ctx->sm_count));
+    if (bn == 128) e = LaunchFor<128, 1>(out, ma, mb, a, idesc, grid, stream);
+    else e = LaunchFor<64, 1>(out, ma, mb, a, idesc, grid, stream);
   }
   if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_gemm (tcgen05) launch: %s", cudaGetErrorString(e)));
   return EndLaunch(ctx, "b200_gemm (tcgen05)");

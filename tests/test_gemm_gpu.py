@@ -243,3 +243,25 @@ def test_config2_large_m_properties(m):
     lin1 = p.blas.matmul(ad, bd)
     lin2 = p.blas.matmul(ad * 2, bd)
     assert torch.equal(lin2, lin1 * 2)
+
+
+@pytest.mark.parametrize("m,n,k,batch,ta,tb", [
+    (8, 16, 16, 5, False, True), (777, 777, 128, 3, False, True), (130, 72, 64, 7, True, False), (257, 264, 320, 2, False, False),
+    (384, 512, 192, 4, True, False)])
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+def test_tcgen05_batched(m, n, k, batch, ta, tb, dt):
+    """Batches as the third dimension of the TMA maps; odd output rows, both tile shapes, a broadcast operand."""
+    r = lambda c: -c % 8    # noqa: E731  padding that keeps the operands' rows 16-byte aligned
+    if (r(m if ta else k), r(k if tb else n)) == (0, 0):
+        run_case(m, n, k, batch=batch, ta=ta, tb=tb, dt_in=dt, alpha=0.5)
+        run_case(m, n, k, batch=batch, ta=ta, tb=tb, dt_in=dt, broadcast_b=True, bias=True, act=3, aux=True)
+    run_case(m, n, k, batch=batch, ta=ta, tb=tb, dt_in=dt, pad=8, beta=0.5)
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k,batch,pad", [(515, 517, 257, 1, 0), (1001, 1003, 67, 1, 3), (301, 333, 129, 6, 1), (2048, 1024, 40, 1, 2)])
+def test_tcgen05_unaligned_rows(m, n, k, batch, pad, ta, tb):
+    """Rows that start on odd elements, copied into aligned ones; at least 2^26 multiply-adds, where that route begins."""
+    assert m * n * k * batch >= 2 ** 26
+    run_case(m, n, k, batch=batch, ta=ta, tb=tb, pad=pad, bias=True, act=2)
+    run_case(m, n, k, batch=batch, ta=ta, tb=tb, pad=pad, dt_in="f16", dt_out="f32", beta=0.5, broadcast_b=batch > 1)
