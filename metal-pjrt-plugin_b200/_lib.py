@@ -172,6 +172,29 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native per-call front (host/host.cpp), bound to the loaded library."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        import torch  # noqa: F401  its libraries are what the extension links against
+        from .context import default_context
+        path = os.path.join(HERE, "_host.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with metal-pjrt-plugin_b200/build.py (there is no fallback path)")
+        loader = importlib.machinery.ExtensionFileLoader("_host", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_host", path, loader=loader))
+        loader.exec_module(module)
+        names = ("b200_qmm_run", "b200_gemm", "b200_gemm_force_route", "b200_rownorm", "b200_sample", "b200_decoder_step")
+        module.bind(tuple(C.cast(getattr(lib(), n), C.c_void_p).value for n in names), check, default_context)
+        _host = module
+    return _host
+
+
 def check(status):
     if status != OK:
         raise B200Error(status, lib().b200_last_error().decode("utf-8", "replace"))

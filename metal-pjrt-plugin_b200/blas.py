@@ -7,7 +7,6 @@ import dataclasses
 from typing import Optional
 
 from . import _lib
-from .context import default_context
 
 ACT_NONE, ACT_RELU, ACT_GELU, ACT_SILU = 0, 1, 2, 3
 
@@ -80,25 +79,10 @@ def gemm_work(p: GemmParams):
 def run_steel_gemm(p: GemmParams, epi: Optional[SteelEpilogue] = None, ctx=None, stream=None, route=0):
     """≙ RunSteelGemm / RunGemv: enqueue on the stream, return nothing, raise
     B200Error(INVALID_ARGUMENT / UNIMPLEMENTED / ...) like the absl::Status."""
-    ctx = ctx or default_context(p.c.tensor.device.index or 0)
-    pc = p.to_c()
-    ec = (epi or SteelEpilogue()).to_c()
-    L = _lib.lib()
-    L.b200_gemm_force_route(ctx.handle, route)
-    try:
-        _lib.check(L.b200_gemm(ctx.handle, stream or _lib.current_stream(), C.byref(pc), C.byref(ec)))
-    finally:
-        L.b200_gemm_force_route(ctx.handle, 0)
+    _lib.host().run_steel_gemm(p, epi, ctx, stream, route)
 
 
 def matmul(a, b, bias=None, act=ACT_NONE, out_dtype=None, transpose_b=False, ctx=None):
     """D = act(a @ op(b) + bias) for row-major 2-D tensors (the form XLA's
     GemmRewriter hands the reference as __cublas$lt$matmul)."""
-    import torch
-    m, k = a.shape
-    n = b.shape[0] if transpose_b else b.shape[1]
-    d = torch.empty((m, n), dtype=out_dtype or a.dtype, device=a.device)
-    p = GemmParams(m, n, k, Operand(a, a.stride(0)), Operand(b, b.stride(0), transpose=transpose_b),
-                   Operand(d, d.stride(0)))
-    run_steel_gemm(p, SteelEpilogue(act, bias), ctx)
-    return d
+    return _lib.host().matmul(a, b, bias, act, -1 if out_dtype is None else _lib.dtype_code(out_dtype), transpose_b, ctx)

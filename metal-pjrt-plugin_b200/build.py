@@ -2,15 +2,20 @@
 
     python metal-pjrt-plugin_b200/build.py [--force] [--verbose]
 
+and _host.so (host/host.cpp, g++), the Python front's per-call work in native code, which
+links the torch that holds the tensors.
+
 Objects go to metal-pjrt-plugin_b200/build/, the library next to this file.
 The library links the CUDA runtime statically and nothing else: no PyTorch, no
 NCCL at link time (NCCL is looked up with dlopen when a tensor-parallel group
 is created).
 """
 import concurrent.futures
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -42,8 +47,27 @@ def _compile(src, verbose):
     return src, obj, r
 
 
+def build_host(force=False):
+    src, so = os.path.join(HERE, "host", "host.cpp"), os.path.join(HERE, "_host.so")
+    abi = os.path.join(ROOT, "include", "b200graft.h")
+    if not force and os.path.exists(so) and os.path.getmtime(so) >= max(os.path.getmtime(src), os.path.getmtime(abi)):
+        return so
+    torch = importlib.util.find_spec("torch").submodule_search_locations[0]
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(ROOT, "include"),
+           "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(torch, "include"),
+           "-isystem", os.path.join(torch, "include", "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
+           src, "-L", os.path.join(torch, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-o", so]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on host/host.cpp")
+    return so
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
+    build_host(force)
     hdr = _newest_header()
     todo, objs = [], []
     for src in _sources():

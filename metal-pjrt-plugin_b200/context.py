@@ -14,6 +14,8 @@ class Context:
 
     def close(self):
         if self.handle:
+            if _lib._host is not None:
+                _lib._host.forget(self.handle.value)
             _lib.lib().b200_context_destroy(self.handle)
             self.handle = None
 

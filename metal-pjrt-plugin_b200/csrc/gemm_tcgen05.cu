@@ -239,36 +239,44 @@ __device__ __forceinline__ void addends(const TcArgs& a, const TOut* drow, int c
 // Where byte b of staged row r lies: 16-byte accesses down a column of rows hit different banks.
 __device__ __forceinline__ int staged(int r, int b) { return r * kStagePitch + ((((b >> 4) ^ r) & 7) << 4) + (b & 15); }
 
-// 32 staged rows of 128 bytes -> global, a row (or four rows by 16-byte pieces) per instruction.
-template <typename TOut>
+// 32 staged rows of kBytes (128 or 64) bytes -> global: 16-byte pieces where rows allow them, else one row per
+// instruction in 4-byte words.  A 16-bit row that starts on an odd element is shifted by one (its words then hold the
+// upper half of one staged word and the lower half of the next lane's), which leaves single elements at its ends.
+template <typename TOut, int kBytes>
 __device__ __forceinline__ void store_rows(const uint8_t* st, TOut* out, int64_t ld, int row0, int rows, int col0, int cols, int lane) {
-  constexpr int kCols = 128 / sizeof(TOut);
-  constexpr int kVec = 16 / sizeof(TOut);
+  constexpr int kCols = kBytes / static_cast<int>(sizeof(TOut));
+  constexpr int kVec = 16 / static_cast<int>(sizeof(TOut));
+  constexpr int kPieces = kBytes / 16, kRowsAtOnce = 32 / kPieces;
   const uintptr_t base = reinterpret_cast<uintptr_t>(out);
   if (cols >= kCols && base % 16 == 0 && ld % kVec == 0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = 4 * i + (lane >> 3);
+    for (int i = 0; i < 32 / kRowsAtOnce; ++i) {
+      const int r = kRowsAtOnce * i + lane / kPieces, c = lane % kPieces;
       if (r < rows)
-        *reinterpret_cast<uint4*>(out + static_cast<int64_t>(row0 + r) * ld + col0 + (lane & 7) * kVec) =
-            *reinterpret_cast<const uint4*>(st + staged(r, (lane & 7) * 16));
+        *reinterpret_cast<uint4*>(out + static_cast<int64_t>(row0 + r) * ld + col0 + c * kVec) =
+            *reinterpret_cast<const uint4*>(st + staged(r, c * 16));
     }
-  } else if (sizeof(TOut) == 2 && base % 4 == 0 && ld % 2 == 0) {
-#pragma unroll 4
+  } else if (sizeof(TOut) == 2) {
+    TOut* o0 = out + static_cast<int64_t>(row0) * ld + col0;
+#pragma unroll 8
     for (int r = 0; r < rows; ++r) {
-      TOut* o = out + static_cast<int64_t>(row0 + r) * ld + col0 + 2 * lane;
-      const uint32_t w = *reinterpret_cast<const uint32_t*>(st + staged(r, 4 * lane));
-      if (2 * lane + 1 < cols) *reinterpret_cast<uint32_t*>(o) = w;
-      else if (2 * lane < cols) *o = *reinterpret_cast<const TOut*>(&w);
+      TOut* o = o0 + static_cast<int64_t>(r) * ld;
+      const int odd = static_cast<int>((reinterpret_cast<uintptr_t>(o) >> 1) & 1);
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(st + staged(r, (4 * lane) & (kBytes - 1)));
+      const uint32_t up = __shfl_down_sync(0xffffffffu, w, 1);
+      if (lane < (cols - odd) / 2) *reinterpret_cast<uint32_t*>(o + odd + 2 * lane) = odd ? __byte_perm(w, up, 0x5432) : w;
+    }
+    if (lane < rows) {
+      TOut* o = o0 + static_cast<int64_t>(lane) * ld;
+      const int odd = static_cast<int>((reinterpret_cast<uintptr_t>(o) >> 1) & 1);
+      if (odd) o[0] = *reinterpret_cast<const TOut*>(st + staged(lane, 0));
+      if ((cols - odd) & 1) o[cols - 1] = *reinterpret_cast<const TOut*>(st + staged(lane, 2 * (cols - 1)));
     }
   } else {
-#pragma unroll 4
-    for (int r = 0; r < rows; ++r) {
-      TOut* o = out + static_cast<int64_t>(row0 + r) * ld + col0;
-#pragma unroll
-      for (int c = 0; c < kCols; c += 32)
-        if (c + lane < cols) o[c + lane] = *reinterpret_cast<const TOut*>(st + staged(r, (c + lane) * static_cast<int>(sizeof(TOut))));
-    }
+#pragma unroll 8
+    for (int r = 0; r < rows; ++r)
+      if (lane < cols)
+        out[static_cast<int64_t>(row0 + r) * ld + col0 + lane] = *reinterpret_cast<const TOut*>(st + staged(r, lane * static_cast<int>(sizeof(TOut))));
   }
 }
 
@@ -544,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 accumulator_free(acc);
                 drained = true;
               }
-              store_rows<TOut>(st, pass == 0 ? AUX : D, a.ldd, row0, rows, col0, min(kPass, a.n - col0), lane);
+              store_rows<TOut, kPass * static_cast<int>(sizeof(TOut))>(st, pass == 0 ? AUX : D, a.ldd, row0, rows, col0, min(kPass, a.n - col0), lane);
               __syncwarp();
             }
           }
@@ -740,7 +748,11 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
   const int64_t k_iters = CeilDiv(k, BK);
   const int a_rows = ta ? BM : static_cast<int>(std::min<int64_t>(BM, CeilDiv(m, 8) * 8));
   // A k step moves a_rows x 64 of A and bn x 64 of B into an SM at about 0.1 MB/us; the MMAs of a 256-wide
-  // tile take 0.27 us.  epi: tcgen05.ld, the fused epilogue and the stores of one tile, overlapped with the next tile's loop.
+  // tile take 0.27 us.  epi: one tile's epilogue and stores, overlapped with the next tile's loop (measured with K = 64,
+  // 8192 x 8192: 43 / 65 / 74 us for the three shapes, about the write limit of HBM; rows whose 128-byte pieces straddle
+  // lines take twice as long).
+  const int out_size = DtypeSize(p->c.dtype);
+  const bool straddle = (p->c.ld * out_size) % 16 != 0 || !Aligned(p->c.ptr, 16);
   auto waves_cost = [&](int64_t tiles, int64_t slots, double t_iter, double epi) {
     return static_cast<double>(CeilDiv(tiles, slots)) * std::max(k_iters * t_iter, epi) + epi;
   };
@@ -749,11 +761,11 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
   {
     const int pairs = ResidentClustersFor<256, 2>(p->c.dtype, 1);
     const int64_t tiles = CeilDiv(m, 2 * BM) * CeilDiv(n, 256) * batch;
-    if (pairs > 0 && m > BM) best = waves_cost(tiles, pairs, 0.39, 2.5), group = 2;
+    if (pairs > 0 && m > BM) best = waves_cost(tiles, pairs, 0.39, straddle ? 6.6 : 3.0), group = 2;
   }
   for (int cand : {128, 64}) {
     // 64 columns are 128-byte pieces of B's rows, which stream at about 0.8 of the rate of 256-byte ones
-    const double t_iter = (a_rows + cand) * (BK * 2) * (cand == 64 ? 1.25e-5 : 1e-5), epi = cand == 128 ? 1.3 : 0.8;
+    const double t_iter = (a_rows + cand) * (BK * 2) * (cand == 64 ? 1.25e-5 : 1e-5), epi = cand == 128 ? (straddle ? 4.5 : 2.3) : (straddle ? 3.4 : 1.3);
     const int64_t tiles = CeilDiv(m, BM) * CeilDiv(n, cand) * batch;
     const double whole = waves_cost(tiles, ctx->sm_count, t_iter, epi);
     if (whole < best) best = whole, bn = cand, group = 1, split = 1;

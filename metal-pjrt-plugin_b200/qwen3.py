@@ -104,32 +104,7 @@ def linear(x, w, residual=None, out_f32=False, rms_gain=None, eps=1e-6, silu_mul
     fuses the x + linear(...) of the decoder layer; out_f32 gives the LM head's
     f32 logits.  rms_gain fuses linear(rms_norm(x, rms_gain, eps), w) (up to 8
     rows); silu_mul fuses linear(silu(gate) * up, w) for x = [gate | up]."""
-    torch = _torch()
-    ctx = ctx or default_context(x.device.index or 0)
-    bits, group, order, q, s, b, N, K = _describe(w)
-    lead = x.shape[:-1]
-    x2 = x.reshape(-1, 2 * K if silu_mul else K)
-    M = x2.shape[0]
-    n_out = N // 2 if silu_pair else N   # silu_pair: w from interleave_gate_up; the result is silu(gate) * up
-    out = torch.empty((M, n_out), dtype=torch.float32 if out_f32 else torch.bfloat16, device=x.device)
-    p = _lib.QmmParamsC()
-    p.bits, p.group, p.nibble_order = bits, group, order
-    p.epilogue = _lib.QMM_OUT_F32 if out_f32 else (_lib.QMM_ADD_RESIDUAL if residual is not None else _lib.QMM_OUT_BF16)
-    if silu_pair:
-        p.epilogue = _lib.QMM_OUT_SILU_PAIR
-    p.x, p.q = x2.data_ptr(), q.data_ptr()
-    p.scale = s.data_ptr() if s is not None else None
-    p.bias = b.data_ptr() if b is not None else None
-    p.residual = residual.data_ptr() if residual is not None else None
-    p.out = out.data_ptr()
-    p.M, p.N, p.K = M, N, K
-    p.ldx, p.ldo = x2.stride(0) if M > 0 else 0, n_out
-    if rms_gain is not None:
-        p.prologue, p.eps, p.prologue_gain = _lib.QMM_PRO_RMSNORM, eps, rms_gain.data_ptr()
-    elif silu_mul:
-        p.prologue = _lib.QMM_PRO_SILU_MUL
-    _lib.check(_lib.lib().b200_qmm_run(ctx.handle, stream or _lib.current_stream(), C.byref(p)))
-    return out.reshape(*lead, n_out)
+    return _lib.host().linear(x, w, residual, out_f32, rms_gain, eps, silu_mul, silu_pair, ctx, stream)
 
 
 def qmm_plan(M, N, K, bits=4, group=64):
@@ -146,13 +121,7 @@ def sample(logits, uniform=None, *, temperature=0.0, top_k=0, top_p=1.0, ctx=Non
     """≙ sample (qwen3.py:395-418): next token int32 [B] from f32 logits [B, V] on the device;
     temperature 0 is greedy.  `uniform` (f32 [B] in [0, 1), device) replaces the reference's
     PRNG key: the categorical draw is the inverse CDF at that number."""
-    torch = _torch()
-    ctx = ctx or default_context(logits.device.index or 0)
-    B, V = logits.shape
-    out = torch.empty((B,), dtype=torch.int32, device=logits.device)
-    _lib.check(_lib.lib().b200_sample(ctx.handle, stream or _lib.current_stream(), _lib.ptr(logits.contiguous()), B, V,
-                                      float(temperature), int(top_k), float(top_p), _lib.ptr(uniform), _lib.ptr(out)))
-    return out
+    return _lib.host().sample(logits, uniform, temperature, top_k, top_p, ctx, stream)
 
 
 def init_cache(cfg, batch, max_len, device="cuda"):
@@ -198,13 +167,11 @@ class Decoder:
     def step(self, tokens, pos, logits=None, stream=None):
         """tokens int32 [B] (device), pos int32 [1] (device). Returns f32 logits
         [B, V]; with tp [world, B, V/world] (rank-major)."""
-        torch = _torch()
-        B = tokens.shape[0]
         if logits is None:
+            torch, B = _torch(), tokens.shape[0]
             shape = (B, self.cfg["vocab"]) if self.world == 1 else (self.world, B, self.cfg["vocab"])
             logits = torch.empty(shape, dtype=torch.float32, device=tokens.device)
-        _lib.check(_lib.lib().b200_decoder_step(self.handle, stream or _lib.current_stream(), _lib.ptr(tokens),
-                                                _lib.ptr(pos), _lib.ptr(logits), B))
+        _lib.host().decoder_step(self.handle, tokens, pos, logits, stream)
         return logits
 
     def launches_per_step(self, batch):
