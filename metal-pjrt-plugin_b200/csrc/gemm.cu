@@ -16,10 +16,13 @@
 //   SIMT     - the general tile kernel below: every dtype, transpose, stride,
 //              batch and beta; true f32 arithmetic for f32 operands (tensor
 //              cores have no f32 multiply, and the f32 block must hold rtol 1e-5).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
 
+namespace cg = cooperative_groups;
 using namespace b200;
 
 namespace b200 {
@@ -50,97 +53,217 @@ struct SimtArgs {
   int ta, tb;
   float alpha, beta;
   int act;
+  int split;           // CTAs of a cluster along K
 };
 
-// 64x64 output tile, 16-wide K steps, 256 threads with a 4x4 micro-tile each.
-template <typename TIn, typename TOut>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const SimtArgs p) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
+// d += {a, a} * {b0, b1}: two IEEE multiply-adds per lane in one instruction, so that the FMA pipes are kept busy
+// with half of the issue slots and the rest go to loads.
+__device__ __forceinline__ void fma_pair(float2& d, float a, const float2& b) {
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%0, %1};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "+f"(d.x), "+f"(d.y)
+      : "f"(a), "f"(b.x), "f"(b.y));
+}
+
+// One shape of the tile kernel: a BM x BN tile by KG groups of threads, TM x TN values a thread; a group takes its own
+// part of every BK-deep step.
+template <int BM_, int BN_, int TM_, int TN_, int KG_, int BK_>
+struct Tile {
+  static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KG = KG_, BK = BK_;
+  static constexpr int kGroup = (BM / TM) * (BN / TN);
+  static constexpr int kThreads = kGroup * KG;
+  static constexpr int kPitchA = BM + 4, kPitchB = BN + 4;   // floats; keeps 16-byte reads aligned
+  static constexpr int kBuffer = BK * (kPitchA + kPitchB);   // floats of one of the two steps held
+  static constexpr size_t kSmem = sizeof(float) * (2 * kBuffer > KG * BM * BN ? 2 * kBuffer : KG * BM * BN);
+  static constexpr int kLoadsA = BM * BK / kThreads, kLoadsB = BN * BK / kThreads;
+  static_assert(BM * BK % kThreads == 0 && BN * BK % kThreads == 0 && kThreads % BK == 0 && kThreads % BM == 0 && kThreads % BN == 0, "");
+};
+// Large products: 8 x 8 values a thread (a step of k costs 4 shared loads of 16 bytes for 32 paired multiply-adds).
+using Large = Tile<128, 128, 8, 8, 1, 16>;
+// Products whose 128 x 128 tiles leave SMs idle: two groups of four warps on a 64 x 64 tile.
+using Medium = Tile<64, 64, 4, 8, 2, 32>;
+// Few rows: eight groups of two warps, each with its own part of k.
+using Few = Tile<16, 64, 4, 4, 8, 64>;
+
+// One thread's share of a step of an operand: `kLoads` values, along the operand's contiguous dimension first.
+// OUTER: rows of op(A) or columns of op(B); BYK: k is the contiguous dimension.
+template <typename TIn, int OUTER, int BK, int THREADS, int LOADS>
+struct Loader {
+  const TIn* p;
+  int64_t step, next;   // elements between a thread's values, between steps of k
+  unsigned inside;      // bit i: value i lies inside the matrix's outer dimension
+  int kk, kk_step;
+  __device__ __forceinline__ Loader(const TIn* base, int64_t ld, bool by_k, int outer0, int outer_size, int k0, int tid) {
+    const int o = by_k ? tid / BK : tid % OUTER;
+    const int o_step = by_k ? THREADS / BK : 0;
+    kk = by_k ? tid % BK : tid / OUTER;
+    kk_step = by_k ? 0 : THREADS / OUTER;
+    p = base + (by_k ? static_cast<int64_t>(outer0 + o) * ld + k0 + kk : static_cast<int64_t>(k0 + kk) * ld + outer0 + o);
+    step = (by_k ? o_step : kk_step) * ld;
+    next = by_k ? BK : BK * ld;
+    inside = 0;
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i) inside |= (outer0 + o + i * o_step < outer_size ? 1u : 0u) << i;
+  }
+  __device__ __forceinline__ void load(int k_left, float (&v)[LOADS]) {   // k_left: values of k from this step on
+#pragma unroll
+    for (int i = 0; i < LOADS; ++i)
+      v[i] = ((inside >> i) & 1u) != 0 && kk + i * kk_step < k_left ? load_as_f32<TIn>(p + i * step) : 0.0f;
+    p += next;
+  }
+};
+
+// What bounds it: the FMA pipes.  Steps are double buffered (registers, then shared memory), the values of a thread lie
+// in runs of four along both dimensions, and finished tiles go through shared memory so that rows are stored whole.
+// split > 1: the CTAs of a cluster (along x) take parts of K and add their tiles through distributed shared memory.
+// Sums run in the order of k within a group; groups and CTAs are added in order.
+template <typename TIn, typename TOut, typename T>
+__global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_kernel(const SimtArgs p) {
+  constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, BK = T::BK;
+  extern __shared__ __align__(16) float smem_f[];
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int group = tid / T::kGroup, gt = tid % T::kGroup;
+  const int tx = gt % (BN / TN), ty = gt / (BN / TN);
+  const int rank = static_cast<int>(blockIdx.x) % p.split;
+  const int m0 = blockIdx.y * BM, n0 = static_cast<int>(blockIdx.x) / p.split * BN;
   const int64_t batch = blockIdx.z;
   const TIn* A = static_cast<const TIn*>(p.a) + batch * p.sa;
   const TIn* B = static_cast<const TIn*>(p.b) + batch * p.sb;
+  const int steps = (p.k + BK - 1) / BK;
+  const int s0 = static_cast<int>(static_cast<int64_t>(rank) * steps / p.split), s1 = static_cast<int>(static_cast<int64_t>(rank + 1) * steps / p.split);
+
+  Loader<TIn, BM, BK, T::kThreads, T::kLoadsA> la(A, p.lda, p.ta == 0, m0, p.m, s0 * BK, tid);
+  Loader<TIn, BN, BK, T::kThreads, T::kLoadsB> lb(B, p.ldb, p.tb != 0, n0, p.n, s0 * BK, tid);
+  float va[T::kLoadsA], vb[T::kLoadsB];
+  auto put = [&](float* buf) {
+#pragma unroll
+    for (int i = 0; i < T::kLoadsA; ++i)
+      buf[p.ta == 0 ? la.kk * T::kPitchA + tid / BK + i * (T::kThreads / BK)
+                    : (la.kk + i * (T::kThreads / BM)) * T::kPitchA + tid % BM] = va[i];
+    float* bb = buf + BK * T::kPitchA;
+#pragma unroll
+    for (int i = 0; i < T::kLoadsB; ++i)
+      bb[p.tb != 0 ? lb.kk * T::kPitchB + tid / BK + i * (T::kThreads / BK)
+                   : (lb.kk + i * (T::kThreads / BN)) * T::kPitchB + tid % BN] = vb[i];
+  };
+  float2 acc[TM][TN / 2];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+
+  if (s0 < s1) {
+    la.load(p.k - s0 * BK, va);
+    lb.load(p.k - s0 * BK, vb);
+    put(smem_f);
+  }
+  __syncthreads();
+  for (int s = s0; s < s1; ++s) {
+    const float* buf = smem_f + ((s - s0) & 1) * T::kBuffer;
+    if (s + 1 < s1) {
+      la.load(p.k - (s + 1) * BK, va);
+      lb.load(p.k - (s + 1) * BK, vb);
+    }
+    const float* pa = buf + group * (BK / T::KG) * T::kPitchA + ty * 4;
+    const float* pb = buf + BK * T::kPitchA + group * (BK / T::KG) * T::kPitchB + tx * 4;
+#pragma unroll
+    for (int kk = 0; kk < BK / T::KG; ++kk) {
+      float4 av[TM / 4], bv[TN / 4];
+#pragma unroll
+      for (int i = 0; i < TM / 4; ++i) av[i] = *reinterpret_cast<const float4*>(pa + kk * T::kPitchA + i * (BM / (TM / 4)));
+#pragma unroll
+      for (int j = 0; j < TN / 4; ++j) bv[j] = *reinterpret_cast<const float4*>(pb + kk * T::kPitchB + j * (BN / (TN / 4)));
+#pragma unroll
+      for (int i = 0; i < TM / 4; ++i) {
+        const float a4[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int j = 0; j < TN / 4; ++j) {
+            fma_pair(acc[4 * i + e][2 * j], a4[e], make_float2(bv[j].x, bv[j].y));
+            fma_pair(acc[4 * i + e][2 * j + 1], a4[e], make_float2(bv[j].z, bv[j].w));
+          }
+      }
+    }
+    if (s + 1 < s1) put(smem_f + ((s + 1 - s0) & 1) * T::kBuffer);   // (last read in the step before: the barrier below)
+    __syncthreads();
+  }
+
+  // ---- the groups' tiles -> shared memory [group][BM][BN]
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int r = (i / 4) * (BM / (TM / 4)) + ty * 4 + i % 4;
+#pragma unroll
+    for (int j = 0; j < TN / 4; ++j)
+      *reinterpret_cast<float4*>(smem_f + (group * BM + r) * BN + j * (BN / (TN / 4)) + tx * 4) =
+          make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  if (p.split > 1) cl.sync();
+  else __syncthreads();
   TOut* D = static_cast<TOut*>(p.d) + batch * p.sd;
   TOut* AUX = p.aux ? static_cast<TOut*>(p.aux) + batch * p.sd : nullptr;
-
-  float acc[4][4];
+  for (int e = rank * T::kThreads + tid; e < BM * BN; e += p.split * T::kThreads) {
+    const int gi = m0 + e / BN, gj = n0 + e % BN;
+    if (gi >= p.m || gj >= p.n) continue;
+    float sum = 0.0f;
+    for (int r = 0; r < p.split; ++r) {
+      const float* t = p.split > 1 ? cl.map_shared_rank(smem_f, r) : smem_f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-
-  for (int k0 = 0; k0 < p.k; k0 += BK) {
-    // A tile: BM x BK.  Thread order follows the contiguous dimension of the operand.
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int idx = tid + it * 256;
-      int i, kk;
-      if (p.ta) { i = idx % BM; kk = idx / BM; } else { kk = idx % BK; i = idx / BK; }
-      const int gi = m0 + i, gk = k0 + kk;
-      float v = 0.0f;
-      if (gi < p.m && gk < p.k)
-        v = load_as_f32<TIn>(A + (p.ta ? static_cast<int64_t>(gk) * p.lda + gi : static_cast<int64_t>(gi) * p.lda + gk));
-      As[kk][i] = v;
+      for (int g = 0; g < T::KG; ++g) sum += t[g * BM * BN + e];
     }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int idx = tid + it * 256;
-      int j, kk;
-      if (p.tb) { kk = idx % BK; j = idx / BK; } else { j = idx % BN; kk = idx / BN; }
-      const int gj = n0 + j, gk = k0 + kk;
-      float v = 0.0f;
-      if (gj < p.n && gk < p.k)
-        v = load_as_f32<TIn>(B + (p.tb ? static_cast<int64_t>(gj) * p.ldb + gk : static_cast<int64_t>(gk) * p.ldb + gj));
-      Bs[kk][j] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 bv = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-      const float a4[4] = {av.x, av.y, av.z, av.w};
-      const float b4[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a4[i], b4[j], acc[i][j]);
-    }
-    __syncthreads();
+    const int64_t o = static_cast<int64_t>(gi) * p.ldd + gj;
+    float v = p.alpha * sum;
+    if (p.beta != 0.0f) v += p.beta * load_as_f32<TOut>(D + o);
+    if (p.bias != nullptr) v += load_as_f32<TOut>(static_cast<const TOut*>(p.bias) + gj);
+    if (AUX != nullptr) AUX[o] = store_from_f32<TOut>(v);
+    D[o] = store_from_f32<TOut>(apply_act(p.act, v));
   }
-
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gi = m0 + ty * 4 + i;
-    if (gi >= p.m) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gj = n0 + tx * 4 + j;
-      if (gj >= p.n) continue;
-      const int64_t o = static_cast<int64_t>(gi) * p.ldd + gj;
-      float v = p.alpha * acc[i][j];
-      if (p.beta != 0.0f) v += p.beta * load_as_f32<TOut>(D + o);
-      if (p.bias != nullptr) v += load_as_f32<TOut>(static_cast<const TOut*>(p.bias) + gj);
-      if (AUX != nullptr) AUX[o] = store_from_f32<TOut>(v);
-      D[o] = store_from_f32<TOut>(apply_act(p.act, v));
-    }
-  }
+  if (p.split > 1) cl.sync();   // the peers may still be reading this CTA's tile
 }
 
-template <typename TIn, typename TOut>
-cudaError_t LaunchSimt(const SimtArgs& a, int64_t batch, cudaStream_t stream) {
+template <typename TIn, typename TOut, typename T>
+cudaError_t LaunchTile(const SimtArgs& a, int64_t batch, cudaStream_t stream) {
+  auto kernel = gemm_simt_kernel<TIn, TOut, T>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T::kSmem));
+  if (e != cudaSuccess) return e;
   LaunchCfg lc;
-  lc.grid = dim3(static_cast<unsigned>(CeilDiv(a.n, 64)), static_cast<unsigned>(CeilDiv(a.m, 64)),
+  lc.grid = dim3(static_cast<unsigned>(CeilDiv(a.n, T::BN) * a.split), static_cast<unsigned>(CeilDiv(a.m, T::BM)),
                  static_cast<unsigned>(batch));
-  lc.block = dim3(256);
+  lc.block = dim3(T::kThreads);
+  lc.smem = T::kSmem;
   lc.stream = stream;
   lc.pdl = true;
-  return Launch(lc, gemm_simt_kernel<TIn, TOut>, a);
+  lc.cluster_x = a.split;
+  return Launch(lc, kernel, a);
+}
+
+// The tile by its cost in multiply-adds on the busiest SM, weighted by how well each shape keeps the pipes busy; then,
+// where tiles are too few for the SMs, a split of K.
+template <typename TIn, typename TOut>
+cudaError_t LaunchSimt(SimtArgs a, int64_t batch, int sm_count, cudaStream_t stream) {
+  auto tiles = [&](int bm, int bn) { return CeilDiv(a.m, bm) * CeilDiv(a.n, bn) * batch; };
+  auto cost = [&](int bm, int bn, double weight) { return static_cast<double>(CeilDiv(tiles(bm, bn), sm_count)) * bm * bn * weight; };
+  auto split = [&](int64_t count) {
+    int s = 1;
+    while (s < 8 && count * s * 2 <= sm_count && a.k / (2 * s) >= 256) s *= 2;
+    return s;
+  };
+  const bool tall_ok = CeilDiv(a.m, 16) <= 65535;
+  const double large = cost(128, 128, 1.0), medium = cost(64, 64, 1.15), few = tall_ok ? cost(16, 64, 2.0) : 1e30;
+  if (few < medium && few < large) {
+    a.split = split(tiles(16, 64));
+    return LaunchTile<TIn, TOut, Few>(a, batch, stream);
+  }
+  if (medium < large) {
+    a.split = split(tiles(64, 64));
+    return LaunchTile<TIn, TOut, Medium>(a, batch, stream);
+  }
+  a.split = 1;
+  return LaunchTile<TIn, TOut, Large>(a, batch, stream);
 }
 
 // Copies rows of `cols` 16-bit elements that start anywhere into rows of `dst_words` 32-bit words.  Bound by memory:
@@ -351,11 +474,11 @@ b200_status b200_gemm(b200_context* ctx, b200_stream stream, const b200_gemm_par
   if (CeilDiv(p->m, 64) > 65535) return Fail(B200_UNIMPLEMENTED, "b200_gemm: m too large for the SIMT kernel grid");
   cudaError_t e;
   const int in = p->a.dtype, out = p->c.dtype;
-  if (in == B200_F32) e = LaunchSimt<float, float>(a, p->batch, stream);
-  else if (in == B200_F16 && out == B200_F16) e = LaunchSimt<__half, __half>(a, p->batch, stream);
-  else if (in == B200_F16) e = LaunchSimt<__half, float>(a, p->batch, stream);
-  else if (out == B200_BF16) e = LaunchSimt<__nv_bfloat16, __nv_bfloat16>(a, p->batch, stream);
-  else e = LaunchSimt<__nv_bfloat16, float>(a, p->batch, stream);
+  if (in == B200_F32) e = LaunchSimt<float, float>(a, p->batch, ctx->sm_count, stream);
+  else if (in == B200_F16 && out == B200_F16) e = LaunchSimt<__half, __half>(a, p->batch, ctx->sm_count, stream);
+  else if (in == B200_F16) e = LaunchSimt<__half, float>(a, p->batch, ctx->sm_count, stream);
+  else if (out == B200_BF16) e = LaunchSimt<__nv_bfloat16, __nv_bfloat16>(a, p->batch, ctx->sm_count, stream);
+  else e = LaunchSimt<__nv_bfloat16, float>(a, p->batch, ctx->sm_count, stream);
   if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_gemm launch: %s", cudaGetErrorString(e)));
   return EndLaunch(ctx, "b200_gemm");
 }

@@ -56,6 +56,38 @@ def test_sampling_matches_the_oracle(kw, V):
             assert z[got[r]] >= kth
 
 
+@pytest.mark.parametrize("B,V,k", [(3, 50257, 50), (18, 50257, 50), (19, 50257, 50), (2, 1, 1), (3, 700, 700), (3, 1024, 1), (3, 1025, 1024),
+                                   (3, 8193, 1000), (2, 1 << 19, 40), (33, 2050, 2), (2, 40000, 0), (33, 4099, 0), (2, 131072, 0),
+                                   (2, 1 << 19, 0), (2, 37, 0)])
+def test_shares_of_a_row(B, V, k):
+    """Around the limits of a CTA's share: empty shares, fewer logits than threads, shares beyond shared memory."""
+    rng = np.random.default_rng(V + k)
+    logits = (rng.standard_normal((B, V)) * 3).astype(np.float32)
+    logits[0] = 1.5                                              # one long run of equals
+    if V > 5:
+        logits[1, 5:] = -np.inf
+    u = rng.random(B).astype(np.float32)
+    got = _run(pkg(), logits, u, temperature=0.9, top_k=k)
+    want, margin = sampling.sample(logits, u.astype(np.float64), temperature=0.9, top_k=k)
+    # the largest cumulative sum is V terms of f32: its rounding (below V * 2^-24, in units of the total) decides nothing else
+    sure = margin > max(1e-4, V * 2.0 ** -24)
+    assert np.array_equal(got[sure], want[sure])
+    assert np.all((got >= 0) & (got < V)) and (V <= 5 or got[1] < 5)
+
+
+def test_nan_and_infinite_rows():
+    logits = np.zeros((4, 5000), np.float32)
+    logits[0] = -np.inf
+    logits[1] = np.nan
+    logits[2, 77] = np.inf
+    logits[3, ::2] = -np.nan
+    for kw in (dict(temperature=0.0), dict(temperature=1.0), dict(temperature=1.0, top_k=30), dict(temperature=1.0, top_k=1024, top_p=0.5)):
+        got = _run(pkg(), logits, np.full(4, 0.5, np.float32), **kw)
+        assert np.all((got >= 0) & (got < 5000)), kw
+        if kw["temperature"] == 0.0:
+            assert got[2] == 77 and got[0] == 0
+
+
 def test_refusals():
     import torch
     p = pkg()
