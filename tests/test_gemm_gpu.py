@@ -265,3 +265,14 @@ def test_tcgen05_unaligned_rows(m, n, k, batch, pad, ta, tb):
     assert m * n * k * batch >= 2 ** 26
     run_case(m, n, k, batch=batch, ta=ta, tb=tb, pad=pad, bias=True, act=2)
     run_case(m, n, k, batch=batch, ta=ta, tb=tb, pad=pad, dt_in="f16", dt_out="f32", beta=0.5, broadcast_b=batch > 1)
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(16, 64, 2048, 1), (1, 130, 4100, 1), (17, 63, 600, 2), (15, 4000, 65, 1), (64, 64, 4096, 1), (65, 128, 1031, 1),
+                                         (500, 700, 31, 1), (1665, 1535, 17, 1), (128, 128, 16, 150), (129, 127, 15, 40)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+def test_simt_tiles(m, n, k, batch, ta, tb):
+    """The three tiles of the general kernel at their edges, with and without a split of K over a cluster."""
+    p = pkg()
+    run_case(m, n, k, batch=batch, dt_in="f32", ta=ta, tb=tb, pad=1, alpha=0.5, beta=1.5, bias=True, act=1, aux=True, route=p._lib.ROUTE_SIMT)
+    if batch == 1:
+        run_case(m, n, k, ta=ta, tb=tb, dt_in="bf16", dt_out="f32", route=p._lib.ROUTE_SIMT)
