@@ -66,8 +66,25 @@ struct TcArgs {
                          // other accumulator rows hold is never stored): a few-row product streams B through a deeper ring
   int bcast_a, bcast_b;  // the operand is the same for every batch
   int split;             // CTAs of a cluster along K (grid.y); 1: persistent CTAs, no cluster
+  // WQ: quantised B [n][k] (scales per row and, for int4, offsets)
+  const __nv_bfloat16* scale;
+  const __nv_bfloat16* offset;
+  int scale_ld;          // scales per row: k / 64, or 1
+  int scale_vec;         // eight of them may be loaded at once
   int* status;
 };
+
+// How B arrives: as 16-bit values by TMA, or quantised, widened into the ring by eight more warps.  The packed weights
+// come through a ring of their own (a further warp issues its TMA loads): boxes of 64 bytes of every row, 64-byte swizzle.
+// What bounds a step of a 128 x 256 tile is then the widening, about 300 issue slots per scheduler against 508 cycles of MMAs.
+// (Packed bytes fetched by the widening threads themselves, each its own row, took 1.05 us a step: 32 lines per load
+// instruction, for weights and for scales.)
+enum { kWide = 0, kQ4Seq = 1, kQ4Half = 2, kQ8 = 3 };
+constexpr int kWidenThreads = 256;
+constexpr int kWidenExtra = kWidenThreads + 32;
+constexpr int kRawRing = 48 * 1024;
+constexpr int kRawBoxBytes = 64;
+__host__ __device__ constexpr int RawSlots(int bn) { return kRawRing / (bn * kRawBoxBytes); }
 
 // ---- PTX wrappers --------------------------------------------------------------------
 // One lane of the (converged) warp, known as such to the compiler.
@@ -178,7 +195,7 @@ struct Smem {
   static constexpr int kABytes = BM * BK * 2;        // 16 KB
   static constexpr int kBBytes = kBCols * BK * 2;
   static constexpr int kRing = 192 * 1024;           // cut into as many stages as fit (TcArgs::stages)
-  static constexpr int kTotal = kRing + kStagingBytes + 1024 /* alignment slack */ + 512 /* barriers */;
+  static constexpr int kTotal = kRing + kStagingBytes + 1024 /* alignment slack */ + 768 /* barriers */;
   static_assert(kTotal <= 232448, "shared memory of one CTA");
 };
 
@@ -332,6 +349,35 @@ __device__ __forceinline__ void mbar_arrive_relaxed(uint64_t* bar, uint32_t rank
       : "memory");
 }
 
+// ---- widening of quantised weights: w = q * s (+ b) rounded once to bf16
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// Nibbles r and r + 4 of v as 128 + q, then q * s + b: q * s is exact, so the fused form rounds once.
+__device__ __forceinline__ uint32_t widen_pair(uint32_t v, int r, uint32_t s2, uint32_t b2) {
+  const uint32_t m = and_or(v >> (4 * r), 0x000f000fu, 0x43004300u);
+  uint32_t q, w;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(q) : "r"(m), "r"(0x43004300u));
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(w) : "r"(q), "r"(s2), "r"(b2));
+  return w;
+}
+// Four int8 as two words of bf16.
+__device__ __forceinline__ uint2 widen_bytes(uint32_t v, float s) {
+  const uint32_t u = v ^ 0x80808080u;   // q + 128; as the low bits of 2^23 + (q + 128)
+  float f[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = (__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650 + i)) - 8388736.0f) * s;
+  return make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+}
+
 struct TileAt {
   int b, tm, tn;
 };
@@ -352,8 +398,8 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   return ra;
 }
 
-template <int BN, int CG, typename TOut>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int BN, int CG, typename TOut, int WQ>
+__global__ void __launch_bounds__(kThreads + (WQ ? kWidenExtra : 0), 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                    const uint32_t idesc) {
   using S = Smem<BN, CG>;
@@ -365,7 +411,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* empty = full + kMaxStages;
   uint64_t* tfull = empty + kMaxStages;
   uint64_t* tempty = tfull + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* raw_full = tempty + 2;
+  constexpr int kRawSlots = WQ ? RawSlots(BN) : 1;
+  uint64_t* raw_empty = raw_full + kRawSlots;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + kRawSlots);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int num_tiles = a.tiles_m * a.tiles_n * a.batch;
@@ -382,8 +431,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (tid == 0) {
     for (int s = 0; s < stages; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], WQ ? 1 + kWidenThreads / 32 : 1);
       mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < kRawSlots; ++i) {
+      mbar_init(&raw_full[i], 1);
+      mbar_init(&raw_empty[i], kWidenThreads / 32);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tfull[i], 1);
@@ -419,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           const uint32_t As = smem_u32(smem + s * a.stage_bytes), Bs = As + a_bytes;
           const uint32_t bar = CG == 2 ? cluster_addr(&full[s], 0) : smem_u32(&full[s]);
-          if (rank == 0) mbar_expect_tx(&full[s], CG * a.stage_bytes);
+          if (rank == 0) mbar_expect_tx(&full[s], WQ ? a_bytes : CG * a.stage_bytes);
           if (!a.ta) {
             tma_load_3d<CG>(As, &tmA, ki * BK, row0, ba, bar);                   // [128 m][64 k]
           } else {
@@ -427,7 +480,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int j = 0; j < BM / 64; ++j)                                      // [64 k][64 m] boxes
               tma_load_3d<CG>(As + j * 8192, &tmA, row0 + j * 64, ki * BK, ba, bar);
           }
-          if (a.tb) {
+          if (WQ) {
+            // (B: the widening warps)
+          } else if (a.tb) {
             tma_load_3d<CG>(Bs, &tmB, ki * BK, col0, bb, bar);                   // [n][64 k]
           } else {
 #pragma unroll
@@ -480,6 +535,140 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     __syncwarp();
+  } else if (WQ && warp == 2 + kEpilogueWarps + kWidenThreads / 32) {
+    // ---------------- packed weights (one lane): a box holds kSteps 64-deep steps of every row of the tile
+    constexpr int kSteps = WQ == kQ8 ? 1 : 2;
+    if (elect_one()) {
+      int slot = 0;
+      uint32_t parity = 1;
+      bool ok = true;
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+        const int col0 = tile_at(a, tile).tn * BN;
+        for (int ki = ki_begin; ki < ki_end; ki += kSteps) {
+          if (!mbar_wait_bounded(&raw_empty[slot], parity)) {
+            report_timeout(a.status, 350 + slot);
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&raw_full[slot], BN * kRawBoxBytes);
+          tma_load_2d(smem_u32(smem + stages * a.stage_bytes + slot * BN * kRawBoxBytes), &tmB, ki * (kRawBoxBytes / kSteps), col0,
+                      smem_u32(&raw_full[slot]));
+          if (++slot == kRawSlots) slot = 0, parity ^= 1;
+        }
+      }
+    }
+    __syncwarp();
+  } else if (WQ && warp >= 2 + kEpilogueWarps) {
+    // ---------------- widening warps: a thread owns its part of one row of every 64-deep step (one group of the weights)
+    constexpr int kSteps = WQ == kQ8 ? 1 : 2;
+    constexpr int kPerRow = kWidenThreads / BN;                                // threads of a row
+    constexpr int kBytes = kRawBoxBytes / kSteps / kPerRow;                    // packed bytes of a thread and step
+    constexpr int kPieces = kBytes / 16 > 0 ? kBytes / 16 : 1;
+    const int wt = tid - kThreads, row = wt / kPerRow, part = wt % kPerRow;
+    const uint8_t* raw = smem + stages * a.stage_bytes + row * kRawBoxBytes;
+    int s = 0, slot = 0;
+    uint32_t parity = 1, raw_parity = 0;
+    bool ok = true;
+    for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+      const int64_t n = min(tile_at(a, tile).tn * BN + row, a.n - 1);
+      const uint16_t* sp = reinterpret_cast<const uint16_t*>(a.scale) + n * a.scale_ld;
+      const uint16_t* bp = reinterpret_cast<const uint16_t*>(a.offset) + n * a.scale_ld;
+      const bool one_scale = a.scale_ld == 1;
+      // scales (and offsets) of eight steps at a time, one such block ahead
+      uint4 s8 = make_uint4(0, 0, 0, 0), b8 = s8, s_next = s8, b_next = s8;
+      auto load8 = [&](int kb) {
+        if (!a.scale_vec) return;
+        s_next = __ldg(reinterpret_cast<const uint4*>(sp + kb));
+        if (WQ != kQ8) b_next = __ldg(reinterpret_cast<const uint4*>(bp + kb));
+      };
+      const uint32_t only = one_scale ? __ldg(sp) : 0u;
+      load8(ki_begin & ~7);
+      for (int kb = ki_begin & ~7; kb < ki_end && ok; kb += 8) {
+        s8 = s_next, b8 = b_next;
+        if (kb + 8 < ki_end) load8(kb + 8);
+        const uint32_t sw[4] = {s8.x, s8.y, s8.z, s8.w}, bw[4] = {b8.x, b8.y, b8.z, b8.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int ki = kb + i;
+          if (ki < ki_begin) continue;
+          if (ki >= ki_end || !ok) break;
+          uint32_t s2, b2;   // the scale and the offset, twice
+          if (a.scale_vec) {
+            s2 = __byte_perm(sw[i / 2], 0, (i & 1) ? 0x3232 : 0x1010);
+            b2 = __byte_perm(bw[i / 2], 0, (i & 1) ? 0x3232 : 0x1010);
+          } else {
+            s2 = (one_scale ? only : __ldg(sp + ki)) * 0x10001u;
+            b2 = WQ == kQ8 ? 0u : __ldg(bp + ki) * 0x10001u;
+          }
+          const int in_box = kSteps == 2 ? (ki - ki_begin) & 1 : 0;
+          if (in_box == 0 && !mbar_wait_bounded(&raw_full[slot], raw_parity)) {
+            report_timeout(a.status, 360 + slot);
+            ok = false;
+            break;
+          }
+          uint4 v[kPieces];
+#pragma unroll
+          for (int j = 0; j < kPieces; ++j)
+            v[j] = *reinterpret_cast<const uint4*>(raw + slot * BN * kRawBoxBytes + (((in_box * (4 / kSteps) + part * kPieces + j) ^ ((row >> 1) & 3)) << 4));
+          if (!mbar_wait_bounded(&empty[s], parity)) {
+            report_timeout(a.status, 340 + s);
+            ok = false;
+            break;
+          }
+          uint8_t* dst = smem + s * a.stage_bytes + a.a_rows * (BK * 2) + row * 128;
+          auto put = [&](int c, const uint4& w) { *reinterpret_cast<uint4*>(dst + ((c ^ (row & 7)) << 4)) = w; };   // chunk c: inputs 8 c ..
+          if (WQ == kQ4Seq) {
+#pragma unroll
+            for (int j = 0; j < kPieces; ++j) {
+              const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint32_t p0 = widen_pair(w[e], 0, s2, b2), p1 = widen_pair(w[e], 1, s2, b2);
+                const uint32_t p2 = widen_pair(w[e], 2, s2, b2), p3 = widen_pair(w[e], 3, s2, b2);
+                put(part * (kBytes / 4) + 4 * j + e, make_uint4(__byte_perm(p0, p1, 0x5410), __byte_perm(p2, p3, 0x5410),
+                                                               __byte_perm(p0, p1, 0x7632), __byte_perm(p2, p3, 0x7632)));
+              }
+            }
+          } else if (WQ == kQ4Half) {
+#pragma unroll
+            for (int j = 0; j < kPieces; ++j) {
+              // a byte of the group holds inputs i and i + 32
+              const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+              for (int e = 0; e < 4; e += 2) {
+                uint32_t lo[4], hi[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  const uint32_t p0 = widen_pair(w[e + h], 0, s2, b2), p1 = widen_pair(w[e + h], 1, s2, b2);
+                  const uint32_t p2 = widen_pair(w[e + h], 2, s2, b2), p3 = widen_pair(w[e + h], 3, s2, b2);
+                  lo[2 * h] = __byte_perm(p0, p2, 0x5410), lo[2 * h + 1] = __byte_perm(p0, p2, 0x7632);
+                  hi[2 * h] = __byte_perm(p1, p3, 0x5410), hi[2 * h + 1] = __byte_perm(p1, p3, 0x7632);
+                }
+                const int c = (part * kBytes + 16 * j + 4 * e) / 8;
+                put(c, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+                put(c + 4, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+              }
+            }
+          } else if (WQ == kQ8) {
+            const float sf = bf16_lo(s2);
+#pragma unroll
+            for (int j = 0; j < kPieces; ++j) {
+              const uint2 w0 = widen_bytes(v[j].x, sf), w1 = widen_bytes(v[j].y, sf), w2 = widen_bytes(v[j].z, sf), w3 = widen_bytes(v[j].w, sf);
+              put(part * (kBytes / 8) + 2 * j, make_uint4(w0.x, w0.y, w1.x, w1.y));
+              put(part * (kBytes / 8) + 2 * j + 1, make_uint4(w2.x, w2.y, w3.x, w3.y));
+            }
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[s]);
+          if (++s == stages) s = 0, parity ^= 1;
+          if (in_box == kSteps - 1 || ki + 1 == ki_end) {
+            if (lane == 0) mbar_arrive(&raw_empty[slot]);
+            if (++slot == kRawSlots) slot = 0, raw_parity ^= 1;
+          }
+        }
+      }
+    }
   } else {
     // ---------------- epilogue warps: TMEM lanes 32 q .. 32 q + 31, columns c_lo .. c_lo + BN / 2 - 1
     const int q = warp & 3;
@@ -568,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // tile from all the partial tiles, read through distributed shared memory.
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 2 + kEpilogueWarps) {
       const TileAt t = tile_at(a, blockIdx.x);
       TOut* D = static_cast<TOut*>(a.d) + t.b * a.sd;
       TOut* AUX = a.aux != nullptr ? static_cast<TOut*>(a.aux) + t.b * a.sd : nullptr;
@@ -647,11 +836,27 @@ bool MakeMap(CUtensorMap* map, int dtype, const void* base, int64_t inner, int64
   return r == CUDA_SUCCESS;
 }
 
-template <int BN, int CG, typename TOut>
+}  // namespace
+namespace b200 {
+// A 2-D map over `rows` rows of bytes; boxes of box_bytes (128 or 64: the span of their swizzle) x box_rows.
+bool EncodeByteRows(CUtensorMap* map, const void* base, int64_t row_bytes, int64_t rows, int box_bytes, int box_rows) {
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(row_bytes), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(row_bytes)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_bytes), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t estr[2] = {1, 1};
+  return Encoder() != nullptr &&
+         Encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+}  // namespace b200
+namespace {
+
+template <int BN, int CG, typename TOut, int WQ>
 cudaError_t LaunchTc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, uint32_t idesc, int grid,
                      cudaStream_t stream) {
   static_assert(BM * (BN / CG + 4) * 4 <= Smem<BN, CG>::kRing, "partial tile must fit the ring");
-  auto kernel = gemm_tc_kernel<BN, CG, TOut>;
+  auto kernel = gemm_tc_kernel<BN, CG, TOut, WQ>;
   static std::atomic<uint64_t> ready{0};   // per device: the shared-memory limit is raised
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -663,7 +868,7 @@ cudaError_t LaunchTc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs&
   }
   LaunchCfg lc;
   lc.grid = dim3(CG * grid, a.split, 1);
-  lc.block = dim3(kThreads);
+  lc.block = dim3(kThreads + (WQ ? kWidenExtra : 0));
   lc.smem = Smem<BN, CG>::kTotal;
   lc.stream = stream;
   lc.pdl = true;
@@ -674,18 +879,18 @@ cudaError_t LaunchTc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs&
 
 // How many clusters of `split` CTAs of this kernel the device holds at once (a GPC takes
 // only whole clusters, so this can be well below SMs / split).  Cached per shape of launch.
-template <int BN, int CG, typename TOut>
+template <int BN, int CG, typename TOut, int WQ>
 int ResidentClusters(int split) {
   static std::mutex mu;
   static int cached[9] = {0};
   std::lock_guard<std::mutex> lock(mu);
   if (cached[split] == 0) {
-    auto kernel = gemm_tc_kernel<BN, CG, TOut>;
+    auto kernel = gemm_tc_kernel<BN, CG, TOut, WQ>;
     int n = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<BN, CG>::kTotal) == cudaSuccess) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(16 * CG, split, 1);
-      cfg.blockDim = dim3(kThreads);
+      cfg.blockDim = dim3(kThreads + (WQ ? kWidenExtra : 0));
       cfg.dynamicSmemBytes = Smem<BN, CG>::kTotal;
       cudaLaunchAttribute attr;
       attr.id = cudaLaunchAttributeClusterDimension;
@@ -702,19 +907,54 @@ int ResidentClusters(int split) {
   return cached[split] > 0 ? cached[split] : 0;
 }
 
-template <int BN, int CG>
+template <int BN, int CG, int WQ = kWide>
 int ResidentClustersFor(int out_dtype, int split) {
-  if (out_dtype == B200_F32) return ResidentClusters<BN, CG, float>(split);
-  if (out_dtype == B200_BF16) return ResidentClusters<BN, CG, __nv_bfloat16>(split);
-  return ResidentClusters<BN, CG, __half>(split);
+  if (out_dtype == B200_F32) return ResidentClusters<BN, CG, float, WQ>(split);
+  if (out_dtype == B200_BF16 || WQ != kWide) return ResidentClusters<BN, CG, __nv_bfloat16, WQ>(split);
+  return ResidentClusters<BN, CG, __half, kWide>(split);
 }
 
-template <int BN, int CG>
+template <int BN, int CG, int WQ = kWide>
 cudaError_t LaunchFor(int out_dtype, const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& a, uint32_t idesc, int grid,
                       cudaStream_t stream) {
-  if (out_dtype == B200_F32) return LaunchTc<BN, CG, float>(ma, mb, a, idesc, grid, stream);
-  if (out_dtype == B200_BF16) return LaunchTc<BN, CG, __nv_bfloat16>(ma, mb, a, idesc, grid, stream);
-  return LaunchTc<BN, CG, __half>(ma, mb, a, idesc, grid, stream);
+  if (out_dtype == B200_F32) return LaunchTc<BN, CG, float, WQ>(ma, mb, a, idesc, grid, stream);
+  if (out_dtype == B200_BF16 || WQ != kWide) return LaunchTc<BN, CG, __nv_bfloat16, WQ>(ma, mb, a, idesc, grid, stream);
+  return LaunchTc<BN, CG, __half, kWide>(ma, mb, a, idesc, grid, stream);
+}
+
+// The quantised product: tiles of 128 x 256 or 128 x 128 and the split of K by the same kind of cost model as RunTcgen05.
+constexpr double kWidenStep256 = 0.40, kWidenStep128 = 0.25;   // us per 64-deep step of a tile
+template <int WQ>
+b200_status RunQuantised(b200_context* ctx, cudaStream_t stream, const CUtensorMap& ma, const b200_qmm_params* p, TcArgs a, int out_dtype) {
+  const int64_t k_iters = a.k / BK;
+  int bn = 256, split = 1;
+  double best = 1e30;
+  for (int cand : {256, 128}) {
+    const double t_iter = cand == 256 ? kWidenStep256 : kWidenStep128, epi = cand == 256 ? 4.0 : 2.3;
+    const int64_t tiles = CeilDiv(a.m, BM) * CeilDiv(a.n, cand);
+    const double whole = static_cast<double>(CeilDiv(tiles, ctx->sm_count)) * std::max(k_iters * t_iter, epi) + epi;
+    if (whole < best) best = whole, bn = cand, split = 1;
+    for (int sp = 2; sp <= 8 && cand == 128; sp *= 2) {
+      if (tiles * sp > ctx->sm_count || k_iters / sp < 4) break;
+      if (tiles > ResidentClustersFor<128, 1, WQ>(out_dtype, sp)) continue;
+      const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 1.5 + epi;
+      if (cost < best) best = cost, bn = cand, split = sp;
+    }
+  }
+  a.split = split;
+  a.tiles_n = static_cast<int>(CeilDiv(a.n, bn));
+  a.stage_bytes = (a.a_rows + bn) * BK * 2;
+  a.stages = std::min(kMaxStages, (192 * 1024 - kRawRing) / a.stage_bytes);
+  CUtensorMap mb;
+  if (!EncodeByteRows(&mb, p->q, p->K * p->bits / 8, p->N, kRawBoxBytes, bn))
+    return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: cuTensorMapEncodeTiled refused the weights"));
+  const int64_t tiles = static_cast<int64_t>(a.tiles_m) * a.tiles_n;
+  const uint32_t idesc = make_idesc(1, 0, 0, bn, BM);
+  const int grid = split > 1 ? static_cast<int>(tiles) : static_cast<int>(std::min<int64_t>(tiles, ctx->sm_count));
+  const cudaError_t e = bn == 256 ? LaunchFor<256, 1, WQ>(out_dtype, ma, mb, a, idesc, grid, stream)
+                                  : LaunchFor<128, 1, WQ>(out_dtype, ma, mb, a, idesc, grid, stream);
+  if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm (tcgen05) launch: %s", cudaGetErrorString(e)));
+  return EndLaunch(ctx, "b200_qmm (tcgen05)");
 }
 
 }  // namespace
@@ -823,6 +1063,43 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
   }
   if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_gemm (tcgen05) launch: %s", cudaGetErrorString(e)));
   return EndLaunch(ctx, "b200_gemm (tcgen05)");
+}
+
+// out = x . dequant(W)^T (+ out, under beta = 1) for quantised weights, widened inside the GEMM: the 16-bit weights
+// never exist in memory.  The parameters have passed b200_qmm_validate; false: x does not meet TMA's alignment.
+bool QuantisedGemmSupports(const b200_qmm_params* p) {
+  const int64_t ldx = p->ldx ? p->ldx : p->K;
+  return p->bits != 16 && Encoder() != nullptr && Aligned(p->x, 16) && ldx % 8 == 0 && CeilDiv(p->M, BM) * CeilDiv(p->N, 128) <= INT32_MAX;
+}
+
+b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
+  b200_status s = BeginLaunch(ctx);
+  if (s != B200_OK) return s;
+  TcArgs a = {};
+  const bool f32_out = p->epilogue == B200_QMM_OUT_F32_RAW;
+  a.a_rows = static_cast<int>(std::min<int64_t>(BM, CeilDiv(p->M, 8) * 8));
+  CUtensorMap ma;
+  const int64_t ldx = p->ldx ? p->ldx : p->K;
+  if (!MakeMap(&ma, B200_BF16, p->x, p->K, p->M, ldx, 1, 0, BK, a.a_rows))
+    return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: cuTensorMapEncodeTiled refused x"));
+  a.d = p->out;
+  a.m = static_cast<int>(p->M);
+  a.n = static_cast<int>(p->N);
+  a.k = static_cast<int>(p->K);
+  a.ldd = p->ldo ? p->ldo : p->N;
+  a.alpha = 1.0f;
+  a.beta = p->epilogue == B200_QMM_ADD_RESIDUAL ? 1.0f : 0.0f;
+  a.tb = 1;
+  a.tiles_m = static_cast<int>(CeilDiv(p->M, BM));
+  a.batch = 1;
+  a.scale = static_cast<const __nv_bfloat16*>(p->scale);
+  a.offset = static_cast<const __nv_bfloat16*>(p->bias);
+  a.scale_ld = static_cast<int>(p->K / p->group);
+  a.scale_vec = a.scale_ld % 8 == 0 && Aligned(p->scale, 16) && (p->bits != 4 || Aligned(p->bias, 16));
+  a.status = ctx->dev_status;
+  const int out = f32_out ? B200_F32 : B200_BF16;
+  if (p->bits == 8) return RunQuantised<kQ8>(ctx, stream, ma, p, a, out);
+  return p->nibble_order == 0 ? RunQuantised<kQ4Seq>(ctx, stream, ma, p, a, out) : RunQuantised<kQ4Half>(ctx, stream, ma, p, a, out);
 }
 
 }  // namespace b200

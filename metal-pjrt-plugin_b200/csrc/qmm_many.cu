@@ -1,9 +1,10 @@
-// Weight-only quantised matmul for MORE than 32 rows of x (prefill-sized batches): the weights are
-// dequantised panel by panel into a bf16 workspace that stays in L2 and each panel goes through the
-// tcgen05 GEMM (≙ the reference beyond ROWS_MAX: dequantize(w, dtype), then x @ w.T,
-// examples/llm/qwen3.py:199-230).  HBM sees the quantised weights once; the 4x larger bf16 panel
-// is written and read back inside the 126 MB L2 (a panel is at most 32 MB, and the same buffer is
-// reused for every panel, so its lines are overwritten before they are evicted).
+// Weight-only quantised matmul for MORE than 32 rows of x (prefill-sized batches; ≙ the reference beyond ROWS_MAX:
+// dequantize(w, dtype), then x @ w.T, examples/llm/qwen3.py:199-230).  Two ways:
+//   * the tensor-core GEMM takes the weights as they are and widens them to bf16 on their way into its ring
+//     (gemm_tcgen05.cu): no bf16 copy exists, but every row of 128 x tiles widens them again;
+//   * the weights are dequantised panel by panel into a bf16 workspace and each panel goes through the general GEMM
+//     (PanelsAreFaster says when, and rows of x that TMA cannot read).  A panel is at most 96 MB, so that it stays in the
+//     126 MB L2: 32 MB panels gave GEMMs of less than a wave of tiles (int4 512 x 12288 -> 4096: 136 us, now 87).
 #include <algorithm>
 
 #include "common.cuh"
@@ -13,7 +14,12 @@ using namespace b200;
 
 namespace {
 
-constexpr int64_t kPanelBytes = 32ll << 20;
+constexpr int64_t kPanelBytes = 96ll << 20;
+
+// Many rows of x pay for the copy.  Only sequential int4 has a kernel that writes it at memory speed.  us for the
+// direct form against panels, 4096 -> 24576 and 12288 -> 4096: 256 rows 107 / 61 against 125 / 73, 512 rows 156 / 102
+// against 150 / 87, 1024 rows 285 / 154 against 204 / 104.
+bool PanelsAreFaster(const b200_qmm_params* p) { return p->bits == 4 && p->nibble_order == 0 && p->M > 384; }
 
 // Sequential int4 in groups of 64: one thread per 8 inputs (one word), 16-byte stores.
 __global__ void dequant_int4_seq_kernel(const uint32_t* q, const __nv_bfloat16* scale, const __nv_bfloat16* bias, uint4* out,
@@ -42,6 +48,10 @@ __global__ void dequant_int4_seq_kernel(const uint32_t* q, const __nv_bfloat16* 
 
 namespace b200 {
 
+// gemm_tcgen05.cu
+bool QuantisedGemmSupports(const b200_qmm_params* p);
+b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
+
 b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
   if (p->prologue != B200_QMM_PRO_NONE)
     return Fail(B200_UNIMPLEMENTED, "b200_qmm: the fused input transforms take up to 32 rows (8 for RMSNorm); M = %lld",
@@ -52,10 +62,16 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
   const int64_t ldx = p->ldx ? p->ldx : K, ldo = p->ldo ? p->ldo : N;
   const bool f32_out = p->epilogue == B200_QMM_OUT_F32_RAW;
   const size_t esz = f32_out ? 4 : 2;
+  if (p->epilogue == B200_QMM_ADD_RESIDUAL && p->residual != p->out) {
+    cudaError_t e = cudaMemcpy2DAsync(p->out, ldo * 2, p->residual, ldo * 2, N * 2, M, cudaMemcpyDeviceToDevice, stream);
+    if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: residual copy: %s", cudaGetErrorString(e)));
+  }
+  if (QuantisedGemmSupports(p) && !PanelsAreFaster(p)) return RunQuantisedGemm(ctx, stream, p);
   // bf16 weights need no workspace: one GEMM over the whole matrix
   int64_t panel = N;
   if (p->bits != 16) {
-    panel = std::max<int64_t>(256, (kPanelBytes / (K * 2)) / 256 * 256);
+    // panels of equal height: a short last one is less than a wave of tiles
+    panel = CeilDiv(CeilDiv(N, CeilDiv(N * K * 2, kPanelBytes)), 256) * 256;
     panel = std::min(panel, N);
     const size_t need = static_cast<size_t>(panel) * K * 2;
     std::lock_guard<std::mutex> lock(ctx->mu);
@@ -74,10 +90,6 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
       }
       ctx->qmm_ws_bytes = need;
     }
-  }
-  if (p->epilogue == B200_QMM_ADD_RESIDUAL && p->residual != p->out) {
-    cudaError_t e = cudaMemcpy2DAsync(p->out, ldo * 2, p->residual, ldo * 2, N * 2, M, cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: residual copy: %s", cudaGetErrorString(e)));
   }
   const int64_t row_bytes = p->bits == 4 ? K / 2 : (p->bits == 8 ? K : 2 * K);
   const int64_t spr = p->bits == 16 ? 0 : K / p->group;
