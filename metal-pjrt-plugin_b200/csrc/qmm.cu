@@ -22,7 +22,7 @@
 //     scale/offset are applied in f32;
 //   * the warps' partial tiles are added by rotating epilogue threads; a K split
 //     across CTAs goes through a thread-block cluster's distributed shared memory.
-// More than 32 rows: qmm_many.cu (dequantised panels in L2 + the tensor-core GEMM).
+// 9 to 32 rows: qmm_mid.cu (here only as b200_gemm's few-row route).  More than 32: qmm_many.cu.
 // An alternative route for up to 8 rows on tcgen05: qmm_tc.cu (on request; slower, and why).
 // Tensor-parallel decoders: the `TP` builds of the kernel take part in the push exchange of
 // partial sums (tp.cuh); their slow paths are out of line, because these kernels pay about a
@@ -34,12 +34,15 @@
 #include <map>
 #include <utility>
 
+#include "qmm_frag.cuh"
 #include "qmm_many.cuh"
+#include "qmm_mid.cuh"
 #include "qmm_tc.cuh"
 #include "tp.cuh"
 
 namespace cg = cooperative_groups;
 using namespace b200;
+using namespace b200::qfrag;
 
 namespace {
 
@@ -47,30 +50,6 @@ constexpr int kConsumerWarps = 16;
 constexpr int kConsumerThreads = kConsumerWarps * 32;
 constexpr int kThreads = kConsumerThreads + 32;  // + one producer warp
 constexpr int kCopyBytes = 2048;                 // bytes of one weight row per bulk copy (RT = 1)
-constexpr int kGroupK = 64;
-
-enum Format { kInt4Seq = 0, kInt4Half = 1, kInt8 = 2, kBf16 = 3 };
-
-template <int FMT>
-struct Fmt {
-  static constexpr int kBits = FMT == kInt8 ? 8 : (FMT == kBf16 ? 16 : 4);
-  static constexpr int kPad = kBits == 4 ? 32 : 64;           // keeps the quad reads conflict-free
-  static constexpr int kGroupBytes = kGroupK * kBits / 8;     // 32 / 64 / 128
-};
-
-// Which input (0..63) of a group sits in half `h` of A register `r` (0..7) of
-// quad thread `t`.  x is staged in shared memory in exactly this order.
-template <int FMT>
-__device__ __forceinline__ int kmap(int t, int r, int h) {
-  if (FMT == kInt4Seq) return 16 * t + 8 * (r >> 2) + (r & 3) + 4 * h;
-  if (FMT == kInt4Half) {
-    const int rr = r & 3;
-    return 8 * t + 4 * (r >> 2) + (rr >> 1) + 2 * h + 32 * (rr & 1);
-  }
-  if (FMT == kInt8) return 16 * t + 2 * r + h;
-  return 32 * (r >> 2) + 8 * t + 2 * (r & 3) + h;  // bf16: two 16-byte pieces per thread
-}
-
 struct QmmArgs {
   const uint8_t* q;
   const __nv_bfloat16* scale;
@@ -223,48 +202,15 @@ __device__ __noinline__ void tp_reduce_publish(const uint2* slot, size_t pitch, 
   }
 }
 
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
-}
-
-// v >> log2(2^32 / pow2).  (Written as a multiply-high by a power of two it would run on the FMA
-// pipe, but that instruction measures 4-6 issue cycles per warp on this GPU against about one
-// for a plain shift.)
-__device__ __forceinline__ uint32_t mulhi_shift(uint32_t v, uint32_t pow2) { return v >> (__clz(pow2) + 1); }
-
 // Widens one thread's share of a group (for one weight row) into 8 bf16x2 registers.
 template <int FMT>
 __device__ __forceinline__ void load_a(const uint8_t* row_group_ptr, int t, uint32_t (&a)[8]) {
-  if (FMT == kInt4Seq || FMT == kInt4Half) {
+  if (Fmt<FMT>::kBits == 4) {
     const uint2 w = *reinterpret_cast<const uint2*>(row_group_ptr + 8 * t);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      // the right shifts are multiply-high by a power of two: that instruction runs on the
-      // FMA pipe, which leaves the (half-rate) integer pipe to the lop3s
-      a[r] = lop3_and_or(r == 0 ? w.x : mulhi_shift(w.x, 1u << (32 - 4 * r)), 0x000f000fu, 0x43004300u);  // bf16 (128 + q)
-      a[4 + r] = lop3_and_or(r == 0 ? w.y : mulhi_shift(w.y, 1u << (32 - 4 * r)), 0x000f000fu, 0x43004300u);
-    }
-  } else if (FMT == kInt8) {
-    const uint4 w = *reinterpret_cast<const uint4*>(row_group_ptr + 16 * t);
-    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t u = words[j] ^ 0x80808080u;  // q + 128 in every byte
-      // 2^23 + (q + 128) as f32, minus (2^23 + 128): q exactly, no int->float unit
-      const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)) - 8388736.0f;
-      const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651)) - 8388736.0f;
-      const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)) - 8388736.0f;
-      const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653)) - 8388736.0f;
-      a[2 * j] = pack_bf16(f0, f1);
-      a[2 * j + 1] = pack_bf16(f2, f3);
-    }
+    widen<FMT>(make_uint4(w.x, w.y, 0, 0), make_uint4(0, 0, 0, 0), a);
   } else {
     const uint4 w0 = *reinterpret_cast<const uint4*>(row_group_ptr + 16 * t);
-    const uint4 w1 = *reinterpret_cast<const uint4*>(row_group_ptr + 64 + 16 * t);
-    a[0] = w0.x; a[1] = w0.y; a[2] = w0.z; a[3] = w0.w;
-    a[4] = w1.x; a[5] = w1.y; a[6] = w1.z; a[7] = w1.w;
+    widen<FMT>(w0, FMT == kBf16 ? *reinterpret_cast<const uint4*>(row_group_ptr + 64 + 16 * t) : w0, a);
   }
 }
 
@@ -288,31 +234,12 @@ __device__ __forceinline__ float2 lds64f(uint32_t addr) {
 // offset (the unrolled path keeps these offsets in registers instead of re-deriving them).
 template <int FMT>
 __device__ __forceinline__ void load_a32(uint32_t addr, uint32_t (&a)[8]) {
-  if (FMT == kInt4Seq || FMT == kInt4Half) {
+  if (Fmt<FMT>::kBits == 4) {
     const uint2 w = lds64(addr);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      a[r] = lop3_and_or(r == 0 ? w.x : mulhi_shift(w.x, 1u << (32 - 4 * r)), 0x000f000fu, 0x43004300u);
-      a[4 + r] = lop3_and_or(r == 0 ? w.y : mulhi_shift(w.y, 1u << (32 - 4 * r)), 0x000f000fu, 0x43004300u);
-    }
-  } else if (FMT == kInt8) {
-    const uint4 w = lds128(addr);
-    const uint32_t words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t u = words[j] ^ 0x80808080u;
-      const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)) - 8388736.0f;
-      const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651)) - 8388736.0f;
-      const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)) - 8388736.0f;
-      const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653)) - 8388736.0f;
-      a[2 * j] = pack_bf16(f0, f1);
-      a[2 * j + 1] = pack_bf16(f2, f3);
-    }
+    widen<FMT>(make_uint4(w.x, w.y, 0, 0), make_uint4(0, 0, 0, 0), a);
   } else {
     const uint4 w0 = lds128(addr);
-    const uint4 w1 = lds128(addr + 64);
-    a[0] = w0.x; a[1] = w0.y; a[2] = w0.z; a[3] = w0.w;
-    a[4] = w1.x; a[5] = w1.y; a[6] = w1.z; a[7] = w1.w;
+    widen<FMT>(w0, FMT == kBf16 ? lds128(addr + 64) : w0, a);
   }
 }
 
@@ -1310,15 +1237,12 @@ cudaError_t LaunchFmt(const Plan& pl, const QmmArgs& args, dim3 grid, cudaStream
     case 12:
       if (args.k_per_cta != 64 * kGroupK || pl.split != 1 || !FastPathOk<GROUPED>(args)) return cudaErrorInvalidValue;
       return LaunchOne<FMT, 1, 2, GROUPED, 64>(pl, args, grid, stream);
-    case 22:
-      if (vec) return LaunchOne<FMT, 2, 2, GROUPED, 0, false, true>(pl, args, grid, stream);
-      return LaunchOne<FMT, 2, 2, GROUPED, 0>(pl, args, grid, stream);
-    case 42:
-      if (vec) return LaunchOne<FMT, 4, 2, GROUPED, 0, false, true>(pl, args, grid, stream);
-      return LaunchOne<FMT, 4, 2, GROUPED, 0>(pl, args, grid, stream);
-    case 44:
-      if (vec) return LaunchOne<FMT, 4, 4, GROUPED, 0, false, true>(pl, args, grid, stream);
-      return LaunchOne<FMT, 4, 4, GROUPED, 0>(pl, args, grid, stream);
+    default:   // more than 8 vectors: b200_gemm's few-row route only (b200_qmm: qmm_mid.cu)
+      if constexpr (FMT == kBf16) {
+        if (pl.mb == 2) return vec ? LaunchOne<FMT, 2, 2, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 2, 2, GROUPED, 0>(pl, args, grid, stream);
+        if (pl.rt == 2) return vec ? LaunchOne<FMT, 4, 2, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 4, 2, GROUPED, 0>(pl, args, grid, stream);
+        return vec ? LaunchOne<FMT, 4, 4, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 4, 4, GROUPED, 0>(pl, args, grid, stream);
+      }
   }
   return cudaErrorInvalidValue;
 }
@@ -1393,6 +1317,15 @@ b200_status b200_qmm_plan(const b200_qmm_params* p, int* rows_per_cta, int* spli
     if (batch_blocks) *batch_blocks = static_cast<int>(CeilDiv(p->M, 8));
     return B200_OK;
   }
+  if (p->M > 8) {
+    int rows = 0, slices = 0, mb = 0;
+    s = QmmMidPlan(p, 148, 227 * 1024, &rows, &slices, &mb);
+    if (s != B200_OK) return s;
+    if (rows_per_cta) *rows_per_cta = rows;
+    if (split_k) *split_k = slices;
+    if (batch_blocks) *batch_blocks = mb;
+    return B200_OK;
+  }
   Plan pl;
   s = MakePlan(p, 148, 227 * 1024, &pl);
   if (s != B200_OK) return s;
@@ -1438,6 +1371,7 @@ b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
     if (tp != nullptr && tp->world > 1) return Fail(B200_UNIMPLEMENTED, "b200_qmm: the exchange takes up to 8 rows");
     return QmmManyRows(ctx, stream, p);
   }
+  if (p->M > 8 && (tp == nullptr || tp->world < 1)) return QmmMidRun(ctx, stream, p);   // batched decoding
   const int forced = ctx->qmm_route.load();
   if (p->epilogue == B200_QMM_OUT_SILU_PAIR) {
     Plan chk;
