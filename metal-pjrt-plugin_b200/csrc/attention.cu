@@ -8,7 +8,12 @@
 // all G query heads that share it, and writes an unnormalised partial
 // (sum p v, running max, sum p) to scratch; a second kernel merges the
 // partials.  All K and V bytes of a CTA are requested up front (one DRAM
-// latency per CTA).  In the fused form the kernel also does what precedes
+// latency per CTA).  Both products run on mma.sync with the query heads as the 8-wide operand and the cache bytes, as
+// loaded, as the 16-row one (positions for q.k, head dimensions for p.v): multiply-adds on the FMA pipes, with a shared
+// load for every eight of them, kept an SM busy twice as long as its share of the KV bytes takes.  The f32 probabilities
+// go in as three bf16 terms, which hold all of their 24 bits.  Decoder step (6 layers) at batch 32, position 2048:
+// 1636 -> 1264 us; batch 8, position 777: 661 -> 611; batch 1, position 2048: 380 -> 361.  (Longer runs of chunks per CTA,
+// prefetched, were slower than a CTA per chunk: 1697 -> 1754 us at batch 32.)  In the fused form the kernel also does what precedes
 // attention in the layer (qwen3.py:366-369): per-head RMSNorm and rotate-half
 // RoPE of q from the fused qkv row, and - in the CTA whose slots contain the
 // new position - of k, plus the cache writes of k and v.  That CTA takes the
@@ -48,7 +53,7 @@ struct AttnArgs {
 // i < D/2 (first and second half of the head).
 template <int D>
 __device__ __forceinline__ void norm_rope_head(const __nv_bfloat16* src, const __nv_bfloat16* w, int pos,
-                                               const AttnArgs& a, int lane, float* dst1, float* dst2) {
+                                               const AttnArgs& a, int lane, __nv_bfloat16* dst1, __nv_bfloat16* dst2) {
   constexpr int PAIRS = D / 64;
   float x1[PAIRS], x2[PAIRS];
   float ss = 0.0f;
@@ -72,20 +77,38 @@ __device__ __forceinline__ void norm_rope_head(const __nv_bfloat16* src, const _
                                : static_cast<float>(1.0 / pow(static_cast<double>(a.theta), static_cast<double>(2 * i) / D));
     float sn, cs;
     sincosf(static_cast<float>(pos) * inv_freq, &sn, &cs);
-    dst1[i] = bf16_round(n1 * cs - n2 * sn);
-    dst2[i] = bf16_round(n2 * cs + n1 * sn);
+    dst1[i] = __float2bfloat16_rn(n1 * cs - n2 * sn);
+    dst2[i] = __float2bfloat16_rn(n2 * cs + n1 * sn);
+  }
+}
+
+// The three bf16 terms of eight f32 values, as the operand pairs of two MMAs (pairs of neighbours in a word).
+__device__ __forceinline__ void split3(const float (&p)[8], uint32_t (&t)[3][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a = p[2 * j], b = p[2 * j + 1];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      t[k][j] = pack_bf16(a, b);
+      a -= bf16_lo(t[k][j]);
+      b -= bf16_hi(t[k][j]);
+    }
   }
 }
 
 template <int D, int G>
-__global__ void __launch_bounds__(kThreads) attn_partial_kernel(const AttnArgs a) {
-  constexpr int HALF = D / 2;
-  constexpr int KV4 = HALF / 8;   // 16-byte loads of K per thread (two threads per position)
-  __shared__ __align__(16) float qs[G][2][HALF + 4];
-  __shared__ __align__(16) float sc[G][kChunk];
-  __shared__ float red[G][kThreads / 32];
-  __shared__ float knew[2][HALF + 4];
-  __shared__ float vnew[D];
+__global__ void __launch_bounds__(kThreads, 4) attn_partial_kernel(const AttnArgs a) {
+  // A lane (g = lane / 4, t = lane % 4) holds eight consecutive inputs 8 t .. of every 32 of its rows g and g + 8 and of
+  // its column g: the order of k inside an MMA does not matter as long as both operands share it.
+  constexpr int KB = D / 32;         // blocks of 32 head dimensions (q.k)
+  constexpr int VB = kChunk / 32;    // blocks of 32 positions (p.v)
+  constexpr int DT = D / 64;         // 16-row tiles of head dimensions per warp (p.v)
+  constexpr int QP = D + 32;         // pitch: rows 64 bytes apart modulo 128
+  __shared__ __align__(16) __nv_bfloat16 qs[G][QP];
+  __shared__ __align__(16) float sc[G][kChunk + 8];
+  __shared__ float red[2][G][kThreads / 32];
+  __shared__ __align__(16) __nv_bfloat16 knew[D];
+  __shared__ __nv_bfloat16 vnew[D];
   // Fused form: the position and the cache slots of earlier steps (all below *pos) do not
   // come from the kernel before this one, so they are requested before waiting for it.
   // Plain form: slot *pos itself is read, and the kernel before this one (the cache write
@@ -113,21 +136,39 @@ __global__ void __launch_bounds__(kThreads) attn_partial_kernel(const AttnArgs a
   const int64_t bkv = static_cast<int64_t>(b) * a.kv_heads + kv;
 
   // ---- request every K and V byte of this CTA now ------------------------------------
-  const int p = tid >> 1, half = tid & 1;    // scores: position p, half of the head dim
-  uint4 kreg[KV4];
-  {
-    const bool have = s0 + p < n_old;
-    const uint4* krow = reinterpret_cast<const uint4*>(a.k_cache + (bkv * a.max_len + s0 + p) * D + half * HALF);
+  const int g = lane >> 2, t = lane & 3;
+  const int p0 = warp * 16 + g;              // positions p0 and p0 + 8 of the chunk
+  uint4 kreg[2][KB];
 #pragma unroll
-    for (int v = 0; v < KV4; ++v) kreg[v] = have ? krow[v] : make_uint4(0, 0, 0, 0);
-  }
-  uint4 vreg[kChunk / 8];
-  const __nv_bfloat16* vrow = a.v_cache + (bkv * D + min(tid, D - 1)) * a.max_len + s0;
-  if (a.vec_v && tid < D) {
+  for (int h = 0; h < 2; ++h) {
+    const bool have = s0 + p0 + 8 * h < n_old;
+    const uint4* krow = reinterpret_cast<const uint4*>(a.k_cache + (bkv * a.max_len + s0 + p0 + 8 * h) * D + 8 * t);
 #pragma unroll
-    for (int j = 0; j < kChunk / 8; ++j)
-      vreg[j] = (s0 + 8 * j < n_old) ? *reinterpret_cast<const uint4*>(vrow + 8 * j) : make_uint4(0, 0, 0, 0);
+    for (int v = 0; v < KB; ++v) kreg[h][v] = have ? krow[4 * v] : make_uint4(0, 0, 0, 0);
   }
+  const int d0 = warp * 16 * DT + g;         // head dimensions d0 + 16 i and d0 + 16 i + 8
+  uint4 vreg[DT][2][VB];
+#pragma unroll
+  for (int i = 0; i < DT; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const __nv_bfloat16* vrow = a.v_cache + (bkv * D + d0 + 16 * i + 8 * h) * a.max_len + s0;
+#pragma unroll
+      for (int v = 0; v < VB; ++v) {
+        const int o = 32 * v + 8 * t;
+        if (a.vec_v) {
+          vreg[i][h][v] = s0 + o < n_old ? *reinterpret_cast<const uint4*>(vrow + o) : make_uint4(0, 0, 0, 0);
+        } else {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint16_t* q = reinterpret_cast<const uint16_t*>(vrow + o + 2 * e);
+            w[e] = (s0 + o + 2 * e < n_old ? q[0] : 0u) | (s0 + o + 2 * e + 1 < n_old ? static_cast<uint32_t>(q[1]) << 16 : 0u);
+          }
+          vreg[i][h][v] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+    }
 
   // ---- queries (and, in the owning CTA, the new key and value) -----------------------
   pdl_wait();   // q (or the fused qkv row) is the previous kernel's output
@@ -135,22 +176,19 @@ __global__ void __launch_bounds__(kThreads) attn_partial_kernel(const AttnArgs a
     const int total_heads = a.heads + 2 * a.kv_heads;
     const __nv_bfloat16* row = a.qkv + static_cast<int64_t>(b) * total_heads * D;
     for (int gq = warp; gq < G; gq += kThreads / 32)
-      norm_rope_head<D>(row + static_cast<int64_t>(kv * G + gq) * D, a.q_norm, pos, a, lane, qs[gq][0], qs[gq][1]);
+      norm_rope_head<D>(row + static_cast<int64_t>(kv * G + gq) * D, a.q_norm, pos, a, lane, qs[gq], qs[gq] + D / 2);
     if (owner) {
       if (warp == (G % 4)) {
-        norm_rope_head<D>(row + static_cast<int64_t>(a.heads + kv) * D, a.k_norm, pos, a, lane, knew[0], knew[1]);
+        norm_rope_head<D>(row + static_cast<int64_t>(a.heads + kv) * D, a.k_norm, pos, a, lane, knew, knew + D / 2);
         __syncwarp();
         __nv_bfloat16* kdst = a.k_cache + (bkv * a.max_len + pos) * D;
-        for (int i = lane; i < HALF; i += 32) {
-          kdst[i] = __float2bfloat16_rn(knew[0][i]);
-          kdst[i + HALF] = __float2bfloat16_rn(knew[1][i]);
-        }
+        for (int i = lane; i < D; i += 32) kdst[i] = knew[i];
       } else if (warp == ((G + 1) % 4)) {
         const __nv_bfloat16* vsrc = row + static_cast<int64_t>(a.heads + a.kv_heads + kv) * D;
         __nv_bfloat16* vdst = a.v_cache + bkv * D * a.max_len + pos;
         for (int d = lane; d < D; d += 32) {
           const __nv_bfloat16 v = vsrc[d];
-          vnew[d] = __bfloat162float(v);
+          vnew[d] = v;
           vdst[static_cast<int64_t>(d) * a.max_len] = v;
         }
       }
@@ -158,125 +196,122 @@ __global__ void __launch_bounds__(kThreads) attn_partial_kernel(const AttnArgs a
   } else {
     for (int i = tid; i < G * D; i += kThreads) {
       const int gq = i / D, d = i % D;
-      qs[gq][d / HALF][d % HALF] = __bfloat162float(a.q[(static_cast<int64_t>(b) * a.heads + kv * G + gq) * D + d]);
+      qs[gq][d] = a.q[(static_cast<int64_t>(b) * a.heads + kv * G + gq) * D + d];
     }
   }
   __syncthreads();
 
-  // ---- scores -------------------------------------------------------------------------
-  float dot[G];
+  // ---- scores: rows = positions, columns = heads; c[2 h + j] is position p0 + 8 h, head 2 t + j
+  if (owner) {
 #pragma unroll
-  for (int gq = 0; gq < G; ++gq) dot[gq] = 0.0f;
-  const bool from_smem = owner && s0 + p == pos;
+    for (int h = 0; h < 2; ++h)
+      if (s0 + p0 + 8 * h == pos) {
 #pragma unroll
-  for (int v = 0; v < KV4; ++v) {
-    float kf[8];
-    if (from_smem) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) kf[j] = knew[half][v * 8 + j];
-    } else {
-      const uint32_t w[4] = {kreg[v].x, kreg[v].y, kreg[v].z, kreg[v].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        kf[2 * j] = bf16_lo(w[j]);
-        kf[2 * j + 1] = bf16_hi(w[j]);
+        for (int v = 0; v < KB; ++v) kreg[h][v] = *reinterpret_cast<const uint4*>(knew + 32 * v + 8 * t);
       }
-    }
-#pragma unroll
-    for (int gq = 0; gq < G; ++gq) {
-      const float4 q0 = *reinterpret_cast<const float4*>(&qs[gq][half][v * 8]);
-      const float4 q1 = *reinterpret_cast<const float4*>(&qs[gq][half][v * 8 + 4]);
-      dot[gq] = fmaf(q0.x, kf[0], dot[gq]);
-      dot[gq] = fmaf(q0.y, kf[1], dot[gq]);
-      dot[gq] = fmaf(q0.z, kf[2], dot[gq]);
-      dot[gq] = fmaf(q0.w, kf[3], dot[gq]);
-      dot[gq] = fmaf(q1.x, kf[4], dot[gq]);
-      dot[gq] = fmaf(q1.y, kf[5], dot[gq]);
-      dot[gq] = fmaf(q1.z, kf[6], dot[gq]);
-      dot[gq] = fmaf(q1.w, kf[7], dot[gq]);
-    }
   }
-  float mx[G];
+  float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-  for (int gq = 0; gq < G; ++gq) {
-    dot[gq] += __shfl_xor_sync(0xffffffffu, dot[gq], 1);   // the two halves of the head dim
-    const float s = p < cnt ? dot[gq] * a.scale : -INFINITY;
-    if (half == 0) sc[gq][p] = s;
-    mx[gq] = warp_max(s);
-    if (lane == 0) red[gq][warp] = mx[gq];
+  for (int v = 0; v < KB; ++v) {
+    const uint4 q = g < G ? *reinterpret_cast<const uint4*>(&qs[g < G ? g : 0][32 * v + 8 * t]) : make_uint4(0, 0, 0, 0);
+    mma_bf16_16816(c, kreg[0][v].x, kreg[1][v].x, kreg[0][v].y, kreg[1][v].y, q.x, q.y);
+    mma_bf16_16816(c, kreg[0][v].z, kreg[1][v].z, kreg[0][v].w, kreg[1][v].w, q.z, q.w);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    c[j] = p0 < cnt ? c[j] * a.scale : -INFINITY;
+    c[2 + j] = p0 + 8 < cnt ? c[2 + j] * a.scale : -INFINITY;
+    float m = fmaxf(c[j], c[2 + j]);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (g == 0 && 2 * t + j < G) red[0][2 * t + j][warp] = m;
   }
   __syncthreads();
-  float lsum[G];
 #pragma unroll
-  for (int gq = 0; gq < G; ++gq) {
-    float m = red[gq][0];
-#pragma unroll
-    for (int w = 1; w < kThreads / 32; ++w) m = fmaxf(m, red[gq][w]);
-    mx[gq] = m;
-    float e = 0.0f;
-    if (tid < kChunk) {
-      e = tid < cnt ? expf(sc[gq][tid] - m) : 0.0f;
-      sc[gq][tid] = e;
+  for (int j = 0; j < 2; ++j) {
+    const int head = 2 * t + j;
+    float l = 0.0f;
+    if (head < G) {
+      const float m = fmaxf(fmaxf(red[0][head][0], red[0][head][1]), fmaxf(red[0][head][2], red[0][head][3]));
+      const float e0 = p0 < cnt ? expf(c[j] - m) : 0.0f, e1 = p0 + 8 < cnt ? expf(c[2 + j] - m) : 0.0f;
+      sc[head][p0] = e0;
+      sc[head][p0 + 8] = e1;
+      l = e0 + e1;
     }
-    lsum[gq] = warp_sum(e);
-  }
-  __syncthreads();   // every thread has read the maxima; sc[][] now holds p
 #pragma unroll
-  for (int gq = 0; gq < G; ++gq)
-    if (lane == 0) red[gq][warp] = lsum[gq];
+    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (g == 0 && head < G) red[1][head][warp] = l;
+  }
   __syncthreads();
 
-  // ---- p . v: one output dimension per thread -------------------------------------------
-  float* part = a.scratch + (bkv * a.splits + split) * G * (D + 2);
-  if (tid < D) {
-    float acc[G];
+  // ---- p . v: rows = head dimensions, columns = heads
+  if (s0 + kChunk > n_old) {   // only the chunk that holds the newest position has slots that are not in the cache (yet)
 #pragma unroll
-    for (int gq = 0; gq < G; ++gq) acc[gq] = 0.0f;
-    if (a.vec_v) {
+    for (int i = 0; i < DT; ++i)
 #pragma unroll
-      for (int j = 0; j < kChunk / 8; ++j) {
-        const uint32_t w[4] = {vreg[j].x, vreg[j].y, vreg[j].z, vreg[j].w};
-        float v[8];
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t fresh = owner ? __bfloat16_as_ushort(vnew[d0 + 16 * i + 8 * h]) : 0u;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = (e & 1) ? bf16_hi(w[e >> 1]) : bf16_lo(w[e >> 1]);
-        if (s0 + 8 * j + 8 > n_old) {   // only the chunk that holds the newest position has such slots
+        for (int v = 0; v < VB; ++v) {
+          uint32_t w[4] = {vreg[i][h][v].x, vreg[i][h][v].y, vreg[i][h][v].z, vreg[i][h][v].w};
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const int s = 8 * j + e;
-            if (s0 + s >= n_old) v[e] = (owner && s0 + s == pos) ? vnew[tid] : 0.0f;
+            const int slot = s0 + 32 * v + 8 * t + e;
+            if (slot >= n_old) {
+              const uint32_t x = owner && slot == pos ? fresh : 0u;
+              w[e / 2] = (e & 1) ? (w[e / 2] & 0xffffu) | (x << 16) : (w[e / 2] & 0xffff0000u) | x;
+            }
           }
-        }
-        // the eight probabilities of a head as two 16-byte broadcast reads (the loop is bound by
-        // shared-memory instructions otherwise: one scalar read per multiply-add)
-#pragma unroll
-        for (int gq = 0; gq < G; ++gq) {
-          const float4 p0 = *reinterpret_cast<const float4*>(&sc[gq][8 * j]);
-          const float4 p1 = *reinterpret_cast<const float4*>(&sc[gq][8 * j + 4]);
-          acc[gq] = fmaf(p0.x, v[0], acc[gq]);
-          acc[gq] = fmaf(p0.y, v[1], acc[gq]);
-          acc[gq] = fmaf(p0.z, v[2], acc[gq]);
-          acc[gq] = fmaf(p0.w, v[3], acc[gq]);
-          acc[gq] = fmaf(p1.x, v[4], acc[gq]);
-          acc[gq] = fmaf(p1.y, v[5], acc[gq]);
-          acc[gq] = fmaf(p1.z, v[6], acc[gq]);
-          acc[gq] = fmaf(p1.w, v[7], acc[gq]);
+          vreg[i][h][v] = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
-    } else {
-      for (int s = 0; s < cnt; ++s) {
-        const float v = s0 + s < n_old ? __bfloat162float(vrow[s]) : ((owner && s0 + s == pos) ? vnew[tid] : 0.0f);
-#pragma unroll
-        for (int gq = 0; gq < G; ++gq) acc[gq] = fmaf(sc[gq][s], v, acc[gq]);
-      }
-    }
-#pragma unroll
-    for (int gq = 0; gq < G; ++gq) part[gq * (D + 2) + tid] = acc[gq];
   }
+  float o[DT][4];
+#pragma unroll
+  for (int i = 0; i < DT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+#pragma unroll
+  for (int v = 0; v < VB; ++v) {
+    float pr[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) pr[e] = 0.0f;
+    if (g < G) {
+      const float4 x = *reinterpret_cast<const float4*>(&sc[g < G ? g : 0][32 * v + 8 * t]), y = *reinterpret_cast<const float4*>(&sc[g < G ? g : 0][32 * v + 8 * t + 4]);
+      pr[0] = x.x, pr[1] = x.y, pr[2] = x.z, pr[3] = x.w, pr[4] = y.x, pr[5] = y.y, pr[6] = y.z, pr[7] = y.w;
+    }
+    uint32_t term[3][4];
+    split3(pr, term);
+#pragma unroll
+    for (int k = 2; k >= 0; --k)   // the small terms first
+#pragma unroll
+      for (int i = 0; i < DT; ++i) {
+        mma_bf16_16816(o[i], vreg[i][0][v].x, vreg[i][1][v].x, vreg[i][0][v].y, vreg[i][1][v].y, term[k][0], term[k][1]);
+        mma_bf16_16816(o[i], vreg[i][0][v].z, vreg[i][1][v].z, vreg[i][0][v].w, vreg[i][1][v].w, term[k][2], term[k][3]);
+      }
+  }
+  // An infinite value meets the zero terms of its probability as NaN: such sums are formed again, term by term.
+#pragma unroll
+  for (int i = 0; i < DT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int head = 2 * t + (e & 1), d = d0 + 16 * i + 8 * (e >> 1);
+      if (o[i][e] == o[i][e] || head >= G) continue;
+      const __nv_bfloat16* vrow = a.v_cache + (bkv * D + d) * a.max_len + s0;
+      float sum = 0.0f;
+#pragma unroll 1
+      for (int s = 0; s < cnt; ++s) sum = fmaf(sc[head][s], __bfloat162float(s0 + s < n_old ? vrow[s] : vnew[d]), sum);
+      o[i][e] = sum;
+    }
+  float* part = a.scratch + (bkv * a.splits + split) * G * (D + 2);
+#pragma unroll
+  for (int i = 0; i < DT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int head = 2 * t + (e & 1);
+      if (head < G) part[head * (D + 2) + d0 + 16 * i + 8 * (e >> 1)] = o[i][e];
+    }
   if (tid < G) {
-    float l = 0.0f;
-    for (int w = 0; w < kThreads / 32; ++w) l += red[tid][w];
-    part[tid * (D + 2) + D] = mx[tid];
-    part[tid * (D + 2) + D + 1] = l;
+    part[tid * (D + 2) + D] = fmaxf(fmaxf(red[0][tid][0], red[0][tid][1]), fmaxf(red[0][tid][2], red[0][tid][3]));
+    part[tid * (D + 2) + D + 1] = (red[1][tid][0] + red[1][tid][1]) + (red[1][tid][2] + red[1][tid][3]);
   }
 }
 
