@@ -17,9 +17,9 @@ namespace {
 constexpr int64_t kPanelBytes = 96ll << 20;
 
 // Many rows of x pay for the copy.  Only sequential int4 has a kernel that writes it at memory speed.  us for the
-// direct form against panels, 4096 -> 24576 and 12288 -> 4096: 256 rows 107 / 61 against 125 / 73, 512 rows 156 / 102
-// against 150 / 87, 1024 rows 285 / 154 against 204 / 104.
-bool PanelsAreFaster(const b200_qmm_params* p) { return p->bits == 4 && p->nibble_order == 0 && p->M > 384; }
+// direct form against panels, 4096 -> 24576 and 12288 -> 4096 with cold caches: 256 rows 107 / 61 against 125 / 73, 512 rows
+// 156 / 102 against 150 / 87 (back to back 4096 -> 24576: 154 against 170), 1024 rows 285 / 154 against 204 / 104.
+bool PanelsAreFaster(const b200_qmm_params* p) { return p->bits == 4 && p->nibble_order == 0 && p->M > 512; }
 
 // Sequential int4 in groups of 64: one thread per 8 inputs (one word), 16-byte stores.
 __global__ void dequant_int4_seq_kernel(const uint32_t* q, const __nv_bfloat16* scale, const __nv_bfloat16* bias, uint4* out,

@@ -1,0 +1,83 @@
+"""linear() with 9 rows of x and more at the sizes where its kernels can go wrong: tiles, slices of K, boxes and groups that
+end early, rows that allow no wide loads.  The reference is a float64 product with the f32 weights of dequantize()."""
+import numpy as np
+import pytest
+
+from util import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _weight(p, kind, n, k, seed):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randn((n, k), generator=g, device="cuda") * 0.02
+    if kind == "bf16":
+        return w.to(torch.bfloat16), w.to(torch.bfloat16).double()
+    q = p.qwen3.quantize_int4(w) if kind.startswith("int4") else p.qwen3.quantize_int8(w, 64 if kind == "int8_g64" else None)
+    if kind == "int4_half":   # the reference's split-half bytes of the same values
+        words = q["q4"].cpu().numpy().view(np.uint32)
+        nib = ((words[:, :, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(n, k // 64, 64).astype(np.uint8)
+        q = {"q4h": torch.from_numpy(nib[:, :, :32] | (nib[:, :, 32:] << 4)).cuda(), "s": q["s"], "b": q["b"]}
+    return q, p.qwen3.dequantize(q, torch.float32).double()
+
+
+def _check(p, m, n, k, kind, form="plain", pad=0):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w, w64 = _weight(p, kind, n, k, m)
+    cols = 2 * k if form == "silu" else k
+    x = torch.randn((m, cols + pad), generator=g, device="cuda").to(torch.bfloat16)[:, :cols]
+    a = x.double()
+    if form == "silu":      # bf16 roundings of the sigmoid, gate * sigmoid and the product
+        gate, up = x[:, :k].float(), x[:, k:].float()
+        sig = torch.sigmoid(gate).to(torch.bfloat16).float()
+        a = ((gate * sig).to(torch.bfloat16).float() * up).to(torch.bfloat16).double()
+    res = torch.randn((m, n), generator=g, device="cuda").to(torch.bfloat16) if form == "residual" else None
+    got = p.qwen3.linear(x if pad == 0 else x.contiguous(), w, residual=res, silu_mul=form == "silu").double()
+    v, mag = a @ w64.T, a.abs() @ w64.abs().T
+    want = v + (res.double() if res is not None else 0)
+    # results are rounded to bf16 (2^-8 in all for two roundings); sums of k f32 terms; above 32 rows the weights are bf16 (2^-9)
+    tol = 2.0 ** -8 * (v.abs() + want.abs()) + mag * (k * 2.0 ** -24 + (2.0 ** -9 if m > 32 and kind != "bf16" else 0.0))
+    if form == "silu":      # a sigmoid that lies on the edge of a bf16 step may round the other way: 2^-8 of one factor
+        tol = tol + mag * 2.0 ** -7
+    err = (got - want).abs()
+    assert bool((err <= tol).all()), (kind, form, float((err - tol).max()))
+
+
+@pytest.mark.parametrize("kind", ["int4", "int4_half", "int8", "int8_g64", "bf16"])
+@pytest.mark.parametrize("n,k", [(1, 64), (31, 192), (130, 576), (257, 4160), (4100, 1088), (6144, 4096)])
+def test_batched_edges(n, k, kind):
+    p = pkg()
+    for m in (9, 16, 17, 32, 33, 129, 513):
+        _check(p, m, n, k, kind)
+
+
+@pytest.mark.parametrize("kind", ["int4", "int8", "int8_g64"])
+@pytest.mark.parametrize("m", [9, 24, 40])
+def test_batched_forms(m, kind):
+    p = pkg()
+    _check(p, m, 1000, 2048, kind, form="residual")
+    if m <= 32:
+        _check(p, m, 520, 6144, kind, form="silu")
+
+
+def test_batched_under_capture():
+    """A captured call replays to the same bytes (the slices' scratch is an allocation of the graph)."""
+    import torch
+    p = pkg()
+    w, _ = _weight(p, "int4", 4096, 4096, 1)
+    x = torch.randn((24, 4096), device="cuda").to(torch.bfloat16)
+    want = p.qwen3.linear(x, w)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        p.qwen3.linear(x, w)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = p.qwen3.linear(x, w)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
