@@ -179,8 +179,15 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
       p.bits = 8, p.N = q->size(0), p.K = q->size(1);
     }
     s = &tensor(item(a[1], s_s));
-    if (p.bits == 4) b = &tensor(item(a[1], s_b));
-    else p.group = static_cast<int32_t>(p.K / s->size(1));
+    if (p.bits == 4) {
+      b = &tensor(item(a[1], s_b));
+    } else {
+      if (s->size(1) == 0) {
+        PyErr_SetString(PyExc_ZeroDivisionError, "an int8 weight without scales");
+        throw Raised();
+      }
+      p.group = static_cast<int32_t>(p.K / s->size(1));
+    }
   } else {
     q = &tensor(a[1]);
     p.bits = 16, p.N = q->size(0), p.K = q->size(1);
