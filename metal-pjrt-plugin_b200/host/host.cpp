@@ -166,16 +166,26 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   b200_context* ctx = context(a[8], x);
   b200_qmm_params p = {};
   const at::Tensor *q, *s = nullptr, *b = nullptr;
+  // the sizes below are read off the packed weights, so their rank is part of the format
+  auto packed = [&](PyObject* o, int64_t dims) {
+    const at::Tensor& t = tensor(o);
+    if (t.dim() != dims) {
+      PyErr_Format(PyExc_ValueError, "packed weights of this format have %lld dimensions, got %lld", static_cast<long long>(dims),
+                   static_cast<long long>(t.dim()));
+      throw Raised();
+    }
+    return &t;
+  };
   if (PyDict_Check(a[1])) {
     PyObject* o;
     if ((o = PyDict_GetItemWithError(a[1], s_q4)) != nullptr) {
-      q = &tensor(o);
+      q = packed(o, 2);
       p.bits = 4, p.group = 64, p.N = q->size(0), p.K = q->size(1) * 8;
     } else if ((o = PyDict_GetItemWithError(a[1], s_q4h)) != nullptr) {
-      q = &tensor(o);
+      q = packed(o, 3);
       p.bits = 4, p.group = 64, p.nibble_order = 1, p.N = q->size(0), p.K = q->size(1) * 64;
     } else {
-      q = &tensor(item(a[1], s_q));
+      q = packed(item(a[1], s_q), 2);
       p.bits = 8, p.N = q->size(0), p.K = q->size(1);
     }
     s = &tensor(item(a[1], s_s));
@@ -189,13 +199,17 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
       p.group = static_cast<int32_t>(p.K / s->size(1));
     }
   } else {
-    q = &tensor(a[1]);
+    q = packed(a[1], 2);
     p.bits = 16, p.N = q->size(0), p.K = q->size(1);
   }
   const at::Tensor* residual = tensor_or_none(a[2]);
   const at::Tensor* gain = tensor_or_none(a[4]);
   const bool out_f32 = as_bool(a[3]), silu_mul = as_bool(a[6]), silu_pair = as_bool(a[7]);
   const int64_t width = silu_mul ? 2 * p.K : p.K, n_out = silu_pair ? p.N / 2 : p.N;
+  if (x.numel() != 0 && (x.dim() == 0 || x.size(-1) != width)) {   // (the result has x's leading dimensions)
+    PyErr_Format(PyExc_RuntimeError, "linear: the rows of x must have %lld elements", static_cast<long long>(width));
+    throw Raised();
+  }
   at::Tensor flat;
   const at::Tensor* x2 = &x;
   if (x.dim() != 2 || x.size(1) != width) flat = x.reshape({-1, width}), x2 = &flat;
