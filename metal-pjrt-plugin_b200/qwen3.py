@@ -121,7 +121,7 @@ def sample(logits, uniform=None, *, temperature=0.0, top_k=0, top_p=1.0, ctx=Non
     """≙ sample (qwen3.py:395-418): next token int32 [B] from f32 logits [B, V] on the device;
     temperature 0 is greedy.  `uniform` (f32 [B] in [0, 1), device) replaces the reference's
     PRNG key: the categorical draw is the inverse CDF at that number."""
-    return _lib.host().sample(logits, uniform, temperature, top_k, top_p, ctx, stream)
+    return _lib.host().sample(logits, uniform, float(temperature), int(top_k), float(top_p), ctx, stream)
 
 
 def init_cache(cfg, batch, max_len, device="cuda"):

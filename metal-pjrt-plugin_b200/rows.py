@@ -7,7 +7,7 @@ KIND_RMS, KIND_SOFTMAX, KIND_LOG_SOFTMAX, KIND_LAYERNORM = 0, 1, 2, 3
 
 
 def rownorm(kind, x, gain=None, beta=None, eps=1e-6, out=None, ctx=None, stream=None):
-    return _lib.host().rownorm(kind, x, gain, beta, eps, out, ctx, stream)
+    return _lib.host().rownorm(kind, x, gain, beta, float(eps), out, ctx, stream)
 
 
 def rms_norm(x, w, eps, **kw):

@@ -105,3 +105,13 @@ def test_refusals():
     assert call(1.0, 10, 0.9, None) == L.INVALID_ARGUMENT
     assert call(0.0, 0, 1.0, None) == L.OK
     assert ctx.error() == 0
+
+
+def test_numbers_of_any_type():
+    """top_k, top_p and temperature are numbers: what int() and float() take."""
+    import torch
+    rng = np.random.default_rng(5)
+    logits, u = rng.standard_normal((2, 500)).astype(np.float32), rng.random(2).astype(np.float32)
+    want = _run(pkg(), logits, u, temperature=0.75, top_k=20, top_p=0.5)
+    got = _run(pkg(), logits, u, temperature=np.float32(0.75), top_k=20.0, top_p=torch.tensor(0.5))
+    assert np.array_equal(got, want)
