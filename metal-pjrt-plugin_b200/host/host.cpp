@@ -296,7 +296,7 @@ PyObject* matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* bias = tensor_or_none(a[2]);
   b200_context* ctx = context(a[6], A);
   const bool tb = as_bool(a[5]);
-  if (A.dim() != 2 || B.dim() != 2) {
+  if (A.dim() != 2) {
     PyErr_SetString(PyExc_ValueError, "matmul takes row-major 2-D tensors");
     throw Raised();
   }

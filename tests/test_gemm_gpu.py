@@ -276,3 +276,10 @@ def test_simt_tiles(m, n, k, batch, ta, tb):
     run_case(m, n, k, batch=batch, dt_in="f32", ta=ta, tb=tb, pad=1, alpha=0.5, beta=1.5, bias=True, act=1, aux=True, route=p._lib.ROUTE_SIMT)
     if batch == 1:
         run_case(m, n, k, ta=ta, tb=tb, dt_in="bf16", dt_out="f32", route=p._lib.ROUTE_SIMT)
+
+
+def test_matmul_takes_a_trailing_dimension_of_one():
+    import torch
+    p = pkg()
+    a, b = torch.randn((5, 64), device="cuda"), torch.randn((64, 33), device="cuda")
+    assert torch.equal(p.blas.matmul(a, b[:, :, None]), p.blas.matmul(a, b))
