@@ -116,6 +116,14 @@ struct b200_decoder {
 
 namespace {
 
+// A step's first kernel (the embedding) waits for everything before the step, and no kernel of a step writes a weight.
+QmmCaller CallerOf(const QmmTp* tp) {
+  QmmCaller c;
+  c.tp = tp;
+  c.weights_settled = true;
+  return c;
+}
+
 b200_status Qmm(b200_decoder* d, cudaStream_t stream, const b200_qweight& w, const void* x, void* out, int batch,
                 int64_t N, int64_t K, int epilogue, const void* residual, int prologue = B200_QMM_PRO_NONE,
                 const void* gain = nullptr, const QmmTp* tp = nullptr) {
@@ -136,7 +144,7 @@ b200_status Qmm(b200_decoder* d, cudaStream_t stream, const b200_qweight& w, con
   p.M = batch;
   p.N = N;
   p.K = K;
-  return QmmRunEx(d->ctx, stream, &p, tp);
+  return QmmRunEx(d->ctx, stream, &p, CallerOf(tp));
 }
 
 b200_status ResidualNorm(b200_decoder* d, cudaStream_t stream, const void* gain, int batch) {
@@ -322,7 +330,7 @@ b200_status Enqueue(b200_decoder* d, cudaStream_t stream, const int32_t* tokens,
     p.M = batch;
     p.N = c.vocab;
     p.K = E;
-    B200_TRY(QmmRunEx(ctx, stream, &p, push ? &from_peers : nullptr));
+    B200_TRY(QmmRunEx(ctx, stream, &p, CallerOf(push ? &from_peers : nullptr)));
   }
   if (tp) B200_TRY(TpAllGather(d->tp, stream, d->logits_local, logits, static_cast<int64_t>(batch) * c.vocab, B200_F32));
   return B200_OK;

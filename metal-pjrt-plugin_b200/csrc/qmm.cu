@@ -11,9 +11,9 @@
 //     packed rows into a shared-memory ring with 1-D bulk async copies
 //     (cp.async.bulk + mbarrier), so tens of KB per SM are in flight without
 //     costing registers;
-//   * the weight copies do not depend on the previous kernel, so they are
-//     issued BEFORE griddepcontrol.wait: under programmatic dependent launch
-//     the next product's weights stream while the previous kernel drains;
+//   * where the caller knows that no earlier kernel still writes the weights (a decoder's
+//     step), their copies are issued BEFORE griddepcontrol.wait: under programmatic dependent
+//     launch the next product's weights stream while the previous kernel drains;
 //   * sixteen consumer warps own fixed sets of 64-input groups: nibbles / bytes
 //     are widened to bf16 in registers (one lop3 per two nibbles, 128 + q with
 //     the 128 folded into the offset term) and fed to mma.sync m16n8k16 with the
@@ -63,6 +63,7 @@ struct QmmArgs {
   int k_per_cta;   // K / gridDim.y, a multiple of 64
   int epilogue;
   int stages;
+  int weights_settled;   // see b200::QmmCaller
   int* status;
   // dense-GEMM use (epilogue == kEpilogueGemm): D = act(alpha * acc + bias), aux = pre-activation
   int64_t out_row_stride;  // between weight rows (n)
@@ -375,11 +376,12 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv_kernel(const __grid_constan
   for (int i = tid; i < groups_cta * MP; i += kThreads) xsum[i] = 0.0f;
   __syncthreads();
   if (!solo) cg::this_cluster().sync();   // the peers' barriers exist before anyone arrives on them
+  if (!a.weights_settled) pdl_wait();     // the kernel before may be storing the weights
 
   bool dead = false;  // a bounded wait gave up: skip the work, keep every barrier
 
   if (warp == kConsumerWarps) {
-    // ---------------- producer warp: weights only, independent of earlier kernels
+    // ---------------- producer warp: weights only
     const int first_fill = min(n_units, NS);
     for (int u = 0; u < n_units; ++u) {
       const int ti = u / n_chunks, c = u - ti * n_chunks;
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(kThreads, 1) qgemv_kernel(const __grid_constan
   } else {
     // ---------------- consumer warps
     // Scales and offsets belong to the weights, so the first tile's are fetched
-    // before waiting on the previous kernel; a later tile's are fetched into
+    // before waiting for x; a later tile's are fetched into
     // registers while the tile before it is computed.  Stored packed (scale,
     // offset) as [group][row].
     const int g0 = k_begin / kGroupK;
@@ -1336,7 +1338,7 @@ b200_status b200_qmm_plan(const b200_qmm_params* p, int* rows_per_cta, int* spli
 }
 
 b200_status b200_qmm_run(b200_context* ctx, b200_stream stream, const b200_qmm_params* p) {
-  return b200::QmmRunEx(ctx, stream, p, nullptr);
+  return b200::QmmRunEx(ctx, stream, p, b200::QmmCaller());
 }
 
 }  // extern "C"
@@ -1359,7 +1361,8 @@ static bool TcRouteEnabled() {
   return on;
 }
 
-b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmTp* tp) {
+b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller) {
+  const QmmTp* tp = caller.tp;
   b200_status s = BeginLaunch(ctx);
   if (s != B200_OK) return s;
   s = Validate(p);
@@ -1371,7 +1374,7 @@ b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
     if (tp != nullptr && tp->world > 1) return Fail(B200_UNIMPLEMENTED, "b200_qmm: the exchange takes up to 8 rows");
     return QmmManyRows(ctx, stream, p);
   }
-  if (p->M > 8 && (tp == nullptr || tp->world < 1)) return QmmMidRun(ctx, stream, p);   // batched decoding
+  if (p->M > 8 && (tp == nullptr || tp->world < 1)) return QmmMidRun(ctx, stream, p, caller);   // batched decoding
   const int forced = ctx->qmm_route.load();
   if (p->epilogue == B200_QMM_OUT_SILU_PAIR) {
     Plan chk;
@@ -1383,7 +1386,7 @@ b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
   }
   if ((tp == nullptr || tp->world <= 1) && p->epilogue != B200_QMM_OUT_SILU_PAIR && (forced == 2 || (forced == 0 && TcRouteEnabled())) &&
       QmmTcEligible(ctx, p))
-    return QmmTcRun(ctx, stream, p);
+    return QmmTcRun(ctx, stream, p, caller.weights_settled);
   Plan pl;
   s = MakePlan(p, ctx->sm_count, ctx->max_smem_optin, &pl);
   if (s != B200_OK) return s;
@@ -1408,6 +1411,7 @@ b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
   a.scale_vec = pl.grouped && (a.k_per_cta / kGroupK) % 8 == 0 && a.scale_ld % 8 == 0 && Aligned(p->scale, 16) &&
                 (p->bits != 4 || Aligned(p->bias, 16));
   a.epilogue = p->epilogue;
+  a.weights_settled = caller.weights_settled;
   a.stages = pl.stages;
   a.status = ctx->dev_status;
   a.out_row_stride = a.out_vec_stride = 0;

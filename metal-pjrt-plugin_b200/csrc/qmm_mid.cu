@@ -49,6 +49,7 @@ struct MidArgs {
   int x_vec, scale_vec;
   int prologue, epilogue;
   int slices;
+  int weights_settled;   // see b200::QmmCaller
   int* status;
 };
 
@@ -102,8 +103,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qmm_mid_kernel(const __grid
     mbar_fence_init();
   }
   __syncwarp();
-  // The warp's boxes of all its tiles as one sequence; fetches run a whole ring ahead.  Weights do not depend on earlier
-  // kernels, so the first ones are requested before the wait below.
+  // The warp's boxes of all its tiles as one sequence; fetches run a whole ring ahead.  Weights that no earlier kernel can
+  // still be storing are requested before the wait below.
+  if (!a.weights_settled) pdl_wait();
   int f_tile = tile0, f_box = 0, f_slot = 0;
   auto fetch = [&]() {
     if (f_tile >= a.tiles) return;
@@ -435,7 +437,7 @@ b200_status QmmMidPlan(const b200_qmm_params* p, int sm_count, int max_smem, int
   return B200_OK;
 }
 
-b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
+b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller) {
   const int mb = p->M <= 16 ? 2 : 4;
   const bool grouped = p->bits == 4 || (p->bits == 8 && p->group == 64);
   const int max_smem = ctx->max_smem_optin - kStaticSmem;
@@ -465,6 +467,7 @@ b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_par
   a.scale_vec = grouped && a.scale_ld % 4 == 0 && pl.groups % 4 == 0 && Aligned(p->scale, 8) && (p->bits != 4 || Aligned(p->bias, 8));   // 8-byte loads
   a.prologue = p->prologue;
   a.epilogue = p->epilogue;
+  a.weights_settled = caller.weights_settled;
   a.status = ctx->dev_status;
   void* scratch = nullptr;
   if (pl.slices > 1) {

@@ -1,10 +1,10 @@
 // The quantised matmul for 9 to 32 rows of x (qmm_mid.cu), as seen by qmm.cu.
 #pragma once
-#include "common.cuh"
+#include "tp.cuh"
 
 namespace b200 {
 // Enqueues it (the parameters have passed b200_qmm_validate, 9 <= M <= 32).
-b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
+b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller);
 // Rows of a tile, slices of K and batch blocks that it would use.
 b200_status QmmMidPlan(const b200_qmm_params* p, int sm_count, int max_smem, int* rows, int* slices, int* mb);
 }  // namespace b200

@@ -78,6 +78,7 @@ struct Args {
   float* parts;           // [tile][max_parts][MT][128] partial rows of tiles shared between CTAs
   unsigned* counters;     // [tile] CTAs that have delivered their part
   int max_parts;
+  int weights_settled;   // see b200::QmmCaller
   int* status;
 };
 
@@ -222,12 +223,13 @@ __global__ void __launch_bounds__(kThreads, 1) qmm_tc_kernel(const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (!a.weights_settled) pdl_wait();   // the kernel before may be storing the weights
   pdl_launch_dependents();
   const uint32_t tmem = mi->tmem;
   volatile int* dead = &mi->dead;
 
   if (warp == kConsumerWarps) {
-    // ---- producer: the weights do not depend on the kernel before this one -----------------
+    // ---- producer: the weights ---------------------------------------------------------------
     if (lane == 0) {
       for (int i = 0; i < n_units; ++i) {
         const int s = i % a.slots;
@@ -652,7 +654,7 @@ bool QmmTcEligible(const b200_context* ctx, const b200_qmm_params* p) {
   return true;
 }
 
-b200_status QmmTcRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
+b200_status QmmTcRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, bool weights_settled) {
   using namespace qtc;
   Args a = {};
   a.scale = static_cast<const __nv_bfloat16*>(p->scale);
@@ -681,6 +683,7 @@ b200_status QmmTcRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
     return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: partial-row scratch too small for N=%d K=%d", a.N, a.K);
   a.parts = ctx->qtc_parts;
   a.counters = ctx->qtc_counters;
+  a.weights_settled = weights_settled;
   a.status = ctx->dev_status;
   a.xchunks = std::min(a.chunks_per_tile, static_cast<int>(CeilDiv(a.units, ctas)));
   // a multiple of four slots: a slot then always belongs to the same warpgroup, whose waits on it stay in phase order

@@ -7,5 +7,5 @@ namespace b200 {
 // K a multiple of 256, aligned operands, and a working set that fits one CTA's shared memory.
 bool QmmTcEligible(const b200_context* ctx, const b200_qmm_params* p);
 // Enqueues it (the parameters have been validated and found eligible).
-b200_status QmmTcRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
+b200_status QmmTcRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, bool weights_settled);
 }  // namespace b200

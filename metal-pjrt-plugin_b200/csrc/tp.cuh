@@ -51,7 +51,15 @@ struct QmmTp {
   const void* x_old = nullptr;            // push: residual rows [M, N] the sum is added to
   void* x_out = nullptr;                  // push: where the new residual rows go
 };
-b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmTp* tp);
+// What a caller inside the library knows about a quantised product beside its parameters.
+struct QmmCaller {
+  const QmmTp* tp = nullptr;
+  // The weights were written, and the writes waited for, before the first kernel of the caller's sequence let its
+  // dependents start: the product may request them while the kernel before it still runs.  Anyone else's weights may be
+  // that kernel's output (kernels here let their dependents start before they store), so their product waits first.
+  bool weights_settled = false;
+};
+b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller);
 // Fills the fields above (push and consume sides) from a connected group; false when the exchange is not connected.
 bool TpPushLink(b200_tp* tp, QmmTp* out);
 
