@@ -173,7 +173,6 @@ void b200_context_destroy(b200_context* ctx) {
   if (ctx->dev_status) cudaFree(ctx->dev_status);
   if (ctx->qtc_parts) cudaFree(ctx->qtc_parts);
   if (ctx->qtc_counters) cudaFree(ctx->qtc_counters);
-  if (ctx->qmm_ws) cudaFree(ctx->qmm_ws);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->host_status) cudaFreeHost(ctx->host_status);
   delete ctx;

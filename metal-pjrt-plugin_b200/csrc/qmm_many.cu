@@ -2,9 +2,10 @@
 // dequantize(w, dtype), then x @ w.T, examples/llm/qwen3.py:199-230).  Two ways:
 //   * the tensor-core GEMM takes the weights as they are and widens them to bf16 on their way into its ring
 //     (gemm_tcgen05.cu): no bf16 copy exists, but every row of 128 x tiles widens them again;
-//   * the weights are dequantised panel by panel into a bf16 workspace and each panel goes through the general GEMM
-//     (PanelsAreFaster says when, and rows of x that TMA cannot read).  A panel is at most 96 MB, so that it stays in the
-//     126 MB L2: 32 MB panels gave GEMMs of less than a wave of tiles (int4 512 x 12288 -> 4096: 136 us, now 87).
+//   * the weights are dequantised panel by panel into bf16 scratch and each panel goes through the general GEMM
+//     (PanelsAreFaster says when, and rows of x that TMA cannot read).  A panel is at most 96 MB (or 256 rows), so that it stays in
+//     the 126 MB L2: 32 MB panels gave GEMMs of less than a wave of tiles (int4 512 x 12288 -> 4096: 136 us, now 87).  The scratch
+//     is stream-ordered memory of the context's pool: calls on several streams each have their own, and a graph owns its.
 #include <algorithm>
 
 #include "common.cuh"
@@ -44,53 +45,12 @@ __global__ void dequant_int4_seq_kernel(const uint32_t* q, const __nv_bfloat16* 
   }
 }
 
-}  // namespace
-
-namespace b200 {
-
-// gemm_tcgen05.cu
-bool QuantisedGemmSupports(const b200_qmm_params* p);
-b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
-
-b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
-  if (p->prologue != B200_QMM_PRO_NONE)
-    return Fail(B200_UNIMPLEMENTED, "b200_qmm: the fused input transforms take up to 32 rows (8 for RMSNorm); M = %lld",
-                static_cast<long long>(p->M));
-  if (p->epilogue == B200_QMM_OUT_F32)
-    return Fail(B200_UNIMPLEMENTED, "b200_qmm: above 32 rows the output is bf16, bf16 + residual, or raw f32");
+// The product by panels of `panel` weight rows (the residual rows are in `out` already).
+b200_status RunPanels(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, int64_t panel, void* ws) {
   const int64_t M = p->M, N = p->N, K = p->K;
   const int64_t ldx = p->ldx ? p->ldx : K, ldo = p->ldo ? p->ldo : N;
   const bool f32_out = p->epilogue == B200_QMM_OUT_F32_RAW;
   const size_t esz = f32_out ? 4 : 2;
-  if (p->epilogue == B200_QMM_ADD_RESIDUAL && p->residual != p->out) {
-    cudaError_t e = cudaMemcpy2DAsync(p->out, ldo * 2, p->residual, ldo * 2, N * 2, M, cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: residual copy: %s", cudaGetErrorString(e)));
-  }
-  if (QuantisedGemmSupports(p) && !PanelsAreFaster(p)) return RunQuantisedGemm(ctx, stream, p);
-  // bf16 weights need no workspace: one GEMM over the whole matrix
-  int64_t panel = N;
-  if (p->bits != 16) {
-    // panels of equal height: a short last one is less than a wave of tiles
-    panel = CeilDiv(CeilDiv(N, CeilDiv(N * K * 2, kPanelBytes)), 256) * 256;
-    panel = std::min(panel, N);
-    const size_t need = static_cast<size_t>(panel) * K * 2;
-    std::lock_guard<std::mutex> lock(ctx->mu);
-    if (ctx->qmm_ws_bytes < need) {
-      // grown on first use (not inside a stream capture: reserve by running the shape once before capturing)
-      if (ctx->qmm_ws != nullptr) {
-        cudaStreamSynchronize(stream);
-        cudaFree(ctx->qmm_ws);
-        ctx->qmm_ws = nullptr;
-        ctx->qmm_ws_bytes = 0;
-      }
-      cudaError_t e = cudaMalloc(&ctx->qmm_ws, need);
-      if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: %zu bytes of dequantisation workspace: %s", need, cudaGetErrorString(e));
-      }
-      ctx->qmm_ws_bytes = need;
-    }
-  }
   const int64_t row_bytes = p->bits == 4 ? K / 2 : (p->bits == 8 ? K : 2 * K);
   const int64_t spr = p->bits == 16 ? 0 : K / p->group;
   for (int64_t r0 = 0; r0 < N; r0 += panel) {
@@ -100,7 +60,7 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
     if (p->bits != 16) {
       const __nv_bfloat16* sp = static_cast<const __nv_bfloat16*>(p->scale) + r0 * spr;
       const __nv_bfloat16* bp = p->bits == 4 ? static_cast<const __nv_bfloat16*>(p->bias) + r0 * spr : nullptr;
-      if (p->bits == 4 && p->nibble_order == 0 && Aligned(ctx->qmm_ws, 16)) {
+      if (p->bits == 4 && p->nibble_order == 0 && Aligned(ws, 16)) {
         b200_status s = BeginLaunch(ctx);
         if (s != B200_OK) return s;
         const int64_t words = rows * (K / 8);
@@ -110,15 +70,15 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
         lc.stream = stream;
         lc.pdl = true;
         cudaError_t e = Launch(lc, dequant_int4_seq_kernel, reinterpret_cast<const uint32_t*>(qp), sp, bp,
-                               static_cast<uint4*>(ctx->qmm_ws), words, static_cast<int>(K / 8));
+                               static_cast<uint4*>(ws), words, static_cast<int>(K / 8));
         if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: dequantise launch: %s", cudaGetErrorString(e)));
         s = EndLaunch(ctx, "b200_qmm (dequantise)");
         if (s != B200_OK) return s;
       } else {
-        b200_status s = b200_dequantize(ctx, stream, p->bits, p->group, p->nibble_order, qp, sp, bp, ctx->qmm_ws, rows, K, B200_BF16);
+        b200_status s = b200_dequantize(ctx, stream, p->bits, p->group, p->nibble_order, qp, sp, bp, ws, rows, K, B200_BF16);
         if (s != B200_OK) return s;
       }
-      wmat = ctx->qmm_ws;
+      wmat = ws;
     }
     // out[:, r0 : r0 + rows] = x . W_panel^T
     b200_gemm_params g = {};
@@ -143,6 +103,51 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
     if (s != B200_OK) return s;
   }
   return B200_OK;
+}
+
+}  // namespace
+
+namespace b200 {
+
+// gemm_tcgen05.cu
+bool QuantisedGemmSupports(const b200_qmm_params* p);
+b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
+
+b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
+  if (p->prologue != B200_QMM_PRO_NONE)
+    return Fail(B200_UNIMPLEMENTED, "b200_qmm: the fused input transforms take up to 32 rows (8 for RMSNorm); M = %lld",
+                static_cast<long long>(p->M));
+  if (p->epilogue == B200_QMM_OUT_F32)
+    return Fail(B200_UNIMPLEMENTED, "b200_qmm: above 32 rows the output is bf16, bf16 + residual, or raw f32");
+  const int64_t M = p->M, N = p->N, K = p->K;
+  const int64_t ldo = p->ldo ? p->ldo : N;
+  const bool direct_ok = QuantisedGemmSupports(p);
+  bool direct = direct_ok && !PanelsAreFaster(p);
+  // bf16 weights need no scratch: one GEMM over the whole matrix
+  int64_t panel = N;
+  void* ws = nullptr;
+  if (p->bits != 16 && !direct) {
+    // panels of equal height: a short last one is less than a wave of tiles
+    const int64_t most = std::max<int64_t>(256, kPanelBytes / (2 * K) / 256 * 256);
+    panel = std::min(CeilDiv(CeilDiv(N, CeilDiv(N, most)), 256) * 256, N);
+    const size_t need = static_cast<size_t>(panel) * K * 2;
+    const cudaError_t e = cudaMallocFromPoolAsync(&ws, need, ctx->pool, stream);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      ws = nullptr;
+      if (!direct_ok)
+        return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: %zu bytes of scratch for dequantised weights: %s", need, cudaGetErrorString(e));
+      direct = true;
+    }
+  }
+  b200_status s = B200_OK;
+  if (p->epilogue == B200_QMM_ADD_RESIDUAL && p->residual != p->out) {
+    const cudaError_t e = cudaMemcpy2DAsync(p->out, ldo * 2, p->residual, ldo * 2, N * 2, M, cudaMemcpyDeviceToDevice, stream);
+    if (e != cudaSuccess) s = Stick(ctx, Fail(B200_INTERNAL, "b200_qmm: residual copy: %s", cudaGetErrorString(e)));
+  }
+  if (s == B200_OK) s = direct ? RunQuantisedGemm(ctx, stream, p) : RunPanels(ctx, stream, p, panel, ws);
+  if (ws != nullptr) cudaFreeAsync(ws, stream);
+  return s;
 }
 
 }  // namespace b200

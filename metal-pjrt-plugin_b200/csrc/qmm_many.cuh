@@ -3,7 +3,7 @@
 #include "common.cuh"
 
 namespace b200 {
-// Dequantises the weights panel by panel into the context's bf16 workspace and runs the
-// tensor-core GEMM on each panel.  The parameters have passed b200_qmm_validate.
+// The tensor-core GEMM on weights widened on their way in, or on panels of dequantised ones.  The parameters have passed
+// b200_qmm_validate.
 b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
 }  // namespace b200

@@ -81,3 +81,76 @@ def test_batched_under_capture():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+def _overlapped(p, weights, xs, rounds=6):
+    """The products on one stream per weight, enqueued in turn without a wait between them."""
+    import torch
+    streams = [torch.cuda.Stream() for _ in weights]
+    torch.cuda.synchronize()
+    out = [[] for _ in weights]
+    for _ in range(rounds):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                out[i].append(p.qwen3.linear(xs[i], weights[i]))
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("m,pad", [(600, 0), (100, 1), (24, 0)])
+def test_overlapping_streams(m, pad):
+    """Calls of one context on several streams: each has scratch of its own (panels; panels for rows TMA cannot read; slices of K)."""
+    import torch
+    p = pkg()
+    weights = [_weight(p, "int4", 2048, 4096, i)[0] for i in range(3)]
+    xs = [torch.randn((m, 4096 + pad), device="cuda").to(torch.bfloat16)[:, :4096] for _ in weights]
+    want = [p.qwen3.linear(x, w) for x, w in zip(xs, weights)]
+    for i, got in enumerate(_overlapped(p, weights, xs)):
+        assert all(torch.equal(g, want[i]) for g in got), i
+
+
+def test_overlapping_threads():
+    import threading
+    import torch
+    p = pkg()
+    weights = [_weight(p, "int4", 2048, 4096, i)[0] for i in range(3)]
+    xs = [torch.randn((m, 4096), device="cuda").to(torch.bfloat16) for m in (600, 700, 20)]
+    want = [p.qwen3.linear(x, w) for x, w in zip(xs, weights)]
+    torch.cuda.synchronize()
+    got = [[] for _ in weights]
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(8):
+                got[i].append(p.qwen3.linear(xs[i], weights[i]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(3):
+        assert len(got[i]) == 8 and all(torch.equal(g, want[i]) for g in got[i]), i
+
+
+def test_captured_panels_outlive_larger_calls():
+    """A graph captured without a warm-up call of its shape, replayed after calls that need larger panels."""
+    import torch
+    p = pkg()
+    w, _ = _weight(p, "int4", 1024, 1024, 1)
+    x = torch.randn((600, 1024), device="cuda").to(torch.bfloat16)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = p.qwen3.linear(x, w)
+    big, _ = _weight(p, "int4", 8192, 4096, 2)
+    xb = torch.randn((600, 4096), device="cuda").to(torch.bfloat16)
+    want = p.qwen3.linear(x, w)
+    p.qwen3.linear(xb, big)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        p.qwen3.linear(xb, big)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
