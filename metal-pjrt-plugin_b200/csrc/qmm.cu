@@ -22,7 +22,8 @@
 //     scale/offset are applied in f32;
 //   * the warps' partial tiles are added by rotating epilogue threads; a K split
 //     across CTAs goes through a thread-block cluster's distributed shared memory.
-// 9 to 32 rows: qmm_mid.cu (here only as b200_gemm's few-row route).  More than 32: qmm_many.cu.
+// 9 to 32 rows: qmm_mid.cu (here only as b200_gemm's few-row route, and where there is no memory for its scratch: int8 per
+// channel 12288 -> 4096, 32 rows, takes 70 us here and 29 there).  More than 32: qmm_many.cu.
 // An alternative route for up to 8 rows on tcgen05: qmm_tc.cu (on request; slower, and why).
 // Tensor-parallel decoders: the `TP` builds of the kernel take part in the push exchange of
 // partial sums (tp.cuh); their slow paths are out of line, because these kernels pay about a
@@ -1239,12 +1240,16 @@ cudaError_t LaunchFmt(const Plan& pl, const QmmArgs& args, dim3 grid, cudaStream
     case 12:
       if (args.k_per_cta != 64 * kGroupK || pl.split != 1 || !FastPathOk<GROUPED>(args)) return cudaErrorInvalidValue;
       return LaunchOne<FMT, 1, 2, GROUPED, 64>(pl, args, grid, stream);
-    default:   // more than 8 vectors: b200_gemm's few-row route only (b200_qmm: qmm_mid.cu)
-      if constexpr (FMT == kBf16) {
-        if (pl.mb == 2) return vec ? LaunchOne<FMT, 2, 2, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 2, 2, GROUPED, 0>(pl, args, grid, stream);
-        if (pl.rt == 2) return vec ? LaunchOne<FMT, 4, 2, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 4, 2, GROUPED, 0>(pl, args, grid, stream);
-        return vec ? LaunchOne<FMT, 4, 4, GROUPED, 0, false, true>(pl, args, grid, stream) : LaunchOne<FMT, 4, 4, GROUPED, 0>(pl, args, grid, stream);
-      }
+    // More than 8 vectors: b200_gemm's few-row route, and b200_qmm where qmm_mid.cu has no scratch.
+    case 22:
+      if (vec) return LaunchOne<FMT, 2, 2, GROUPED, 0, false, true>(pl, args, grid, stream);
+      return LaunchOne<FMT, 2, 2, GROUPED, 0>(pl, args, grid, stream);
+    case 42:
+      if (vec) return LaunchOne<FMT, 4, 2, GROUPED, 0, false, true>(pl, args, grid, stream);
+      return LaunchOne<FMT, 4, 2, GROUPED, 0>(pl, args, grid, stream);
+    case 44:
+      if (vec) return LaunchOne<FMT, 4, 4, GROUPED, 0, false, true>(pl, args, grid, stream);
+      return LaunchOne<FMT, 4, 4, GROUPED, 0>(pl, args, grid, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -1374,8 +1379,11 @@ b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_para
     if (tp != nullptr && tp->world > 1) return Fail(B200_UNIMPLEMENTED, "b200_qmm: the exchange takes up to 8 rows");
     return QmmManyRows(ctx, stream, p);
   }
-  if (p->M > 8 && (tp == nullptr || tp->world < 1)) return QmmMidRun(ctx, stream, p, caller);   // batched decoding
   const int forced = ctx->qmm_route.load();
+  if (p->M > 8 && forced != 1 && (tp == nullptr || tp->world < 1)) {   // batched decoding
+    s = QmmMidRun(ctx, stream, p, caller);
+    if (s != B200_RESOURCE_EXHAUSTED) return s;   // without scratch: the streaming kernel, which needs none
+  }
   if (p->epilogue == B200_QMM_OUT_SILU_PAIR) {
     Plan chk;
     b200_status ps = MakePlan(p, ctx->sm_count, ctx->max_smem_optin, &chk);

@@ -62,6 +62,20 @@ def test_batched_forms(m, kind):
         _check(p, m, 520, 6144, kind, form="silu")
 
 
+@pytest.mark.parametrize("kind", ["int4", "int4_half", "int8", "int8_g64", "bf16"])
+def test_batched_without_scratch(kind):
+    """Route 1: 9 to 32 rows on the kernel that needs no scratch."""
+    p = pkg()
+    p.lib().b200_qmm_force_route(p.default_context().handle, 1)
+    try:
+        for m, n, k in ((9, 31, 192), (16, 257, 1088), (17, 130, 576), (32, 4100, 4096), (32, 1000, 12288)):
+            _check(p, m, n, k, kind)
+            _check(p, m, n, k, kind, form="residual")
+        _check(p, 24, 520, 6144, kind, form="silu")
+    finally:
+        p.lib().b200_qmm_force_route(p.default_context().handle, 0)
+
+
 def test_batched_under_capture():
     """A captured call replays to the same bytes (the slices' scratch is an allocation of the graph)."""
     import torch
