@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "decode_stream.cuh"
+#include "qmm_mid.cuh"
 
 using namespace b200;
 
@@ -94,6 +95,11 @@ struct b200_decoder {
   __nv_bfloat16* x2 = nullptr;   // second residual buffer of the push exchange (one CTA writes the new rows while all read the old)
   float *y32 = nullptr, *attn_scratch = nullptr, *logits_local = nullptr, *inv_freq = nullptr;
   __nv_bfloat16* logits_bf16 = nullptr;   // LM head output of the tensor-core route (batches above 8)
+  // sums of the slices of K of any one projection (batches above 8).  Memory of the pool instead would be an allocation node
+  // between every two kernels of the captured step: a graph that a caller's own capture cannot take in, without
+  // the edges that let a projection request its weights early.
+  float* slices = nullptr;
+  size_t slices_floats = 0;
   bool use_graph = true;
   cudaStream_t capture_stream = nullptr;  // graphs are captured here (the caller's stream may be the legacy one)
   // Captured steps, keyed by (batch, logits pointer) and most recently used first.  Tokens and
@@ -117,10 +123,12 @@ struct b200_decoder {
 namespace {
 
 // A step's first kernel (the embedding) waits for everything before the step, and no kernel of a step writes a weight.
-QmmCaller CallerOf(const QmmTp* tp) {
+QmmCaller CallerOf(const b200_decoder* d, const QmmTp* tp) {
   QmmCaller c;
   c.tp = tp;
   c.weights_settled = true;
+  c.scratch = d->slices;
+  c.scratch_floats = d->slices_floats;
   return c;
 }
 
@@ -144,7 +152,7 @@ b200_status Qmm(b200_decoder* d, cudaStream_t stream, const b200_qweight& w, con
   p.M = batch;
   p.N = N;
   p.K = K;
-  return QmmRunEx(d->ctx, stream, &p, CallerOf(tp));
+  return QmmRunEx(d->ctx, stream, &p, CallerOf(d, tp));
 }
 
 b200_status ResidualNorm(b200_decoder* d, cudaStream_t stream, const void* gain, int batch) {
@@ -330,7 +338,7 @@ b200_status Enqueue(b200_decoder* d, cudaStream_t stream, const int32_t* tokens,
     p.M = batch;
     p.N = c.vocab;
     p.K = E;
-    B200_TRY(QmmRunEx(ctx, stream, &p, CallerOf(push ? &from_peers : nullptr)));
+    B200_TRY(QmmRunEx(ctx, stream, &p, CallerOf(d, push ? &from_peers : nullptr)));
   }
   if (tp) B200_TRY(TpAllGather(d->tp, stream, d->logits_local, logits, static_cast<int64_t>(batch) * c.vocab, B200_F32));
   return B200_OK;
@@ -384,6 +392,14 @@ b200_status b200_decoder_create(b200_context* ctx, const b200_decoder_config* cf
                    b200_attention_scratch_bytes(c.max_batch, c.heads, c.head_dim, c.max_len));
   if (e == cudaSuccess && tp != nullptr) e = Alloc(&d->logits_local, B * c.vocab);
   if (e == cudaSuccess && c.max_batch > 8) e = Alloc(&d->logits_bf16, B * c.vocab);
+  if (c.max_batch > 8) {
+    const int64_t shapes[4][2] = {{static_cast<int64_t>(qkv), c.hidden}, {c.hidden, static_cast<int64_t>(c.heads) * c.head_dim},
+                                  {2 * static_cast<int64_t>(c.inter), c.hidden}, {c.hidden, c.inter}};
+    for (int m : {9, c.max_batch})   // (a plan depends on the rows only through up to 16 or more)
+      for (const auto& nk : shapes) d->slices_floats = std::max(d->slices_floats, QmmMidScratchFloats(ctx, 4, 64, m, nk[0], nk[1]));
+    d->slices_floats = std::max<size_t>(d->slices_floats, 1);
+    if (e == cudaSuccess) e = Alloc(&d->slices, d->slices_floats);
+  }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->capture_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = Alloc(&d->inv_freq, static_cast<size_t>(c.head_dim / 2));
   if (e == cudaSuccess) e = Alloc(&d->tokens_buf, B);
@@ -474,7 +490,7 @@ void b200_decoder_destroy(b200_decoder* d) {
                   static_cast<void*>(d->y32), static_cast<void*>(d->attn_scratch),
                   static_cast<void*>(d->logits_local), static_cast<void*>(d->inv_freq),
                   static_cast<void*>(d->logits_bf16), static_cast<void*>(d->x2), static_cast<void*>(d->tokens_buf),
-                  static_cast<void*>(d->pos_buf)})
+                  static_cast<void*>(d->pos_buf), static_cast<void*>(d->slices)})
     if (p != nullptr) cudaFree(p);
   for (void* p : d->pair_storage) cudaFree(p);
   delete d;

@@ -398,6 +398,8 @@ bool MakeMidPlan(int bits, bool grouped, int mb, int64_t N, int64_t K, int sm_co
   return best < 1e30;
 }
 
+size_t PlanScratch(const MidPlan& pl, int mb, int64_t N) { return pl.slices > 1 ? static_cast<size_t>(pl.slices) * N * mb * 8 : 0; }
+
 template <int FMT, int MB, bool GROUPED>
 cudaError_t LaunchMid(const MidPlan& pl, const CUtensorMap& map, const MidArgs& a, int max_smem, cudaStream_t stream) {
   auto kernel = qmm_mid_kernel<FMT, MB, GROUPED>;
@@ -437,6 +439,13 @@ b200_status QmmMidPlan(const b200_qmm_params* p, int sm_count, int max_smem, int
   return B200_OK;
 }
 
+size_t QmmMidScratchFloats(const b200_context* ctx, int bits, int group, int64_t M, int64_t N, int64_t K) {
+  const int mb = M <= 16 ? 2 : 4;
+  MidPlan pl;
+  if (!MakeMidPlan(bits, bits == 4 || (bits == 8 && group == 64), mb, N, K, ctx->sm_count, ctx->max_smem_optin - kStaticSmem, &pl)) return 0;
+  return PlanScratch(pl, mb, N);
+}
+
 b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller) {
   const int mb = p->M <= 16 ? 2 : 4;
   const bool grouped = p->bits == 4 || (p->bits == 8 && p->group == 64);
@@ -469,15 +478,21 @@ b200_status QmmMidRun(b200_context* ctx, cudaStream_t stream, const b200_qmm_par
   a.epilogue = p->epilogue;
   a.weights_settled = caller.weights_settled;
   a.status = ctx->dev_status;
-  void* scratch = nullptr;
+  void* scratch = nullptr;   // to be given back
   if (pl.slices > 1) {
-    // stream-ordered memory of the context's pool (an allocation node under capture)
-    cudaError_t e = cudaMallocFromPoolAsync(&scratch, static_cast<size_t>(pl.slices) * p->N * mb * 8 * sizeof(float), ctx->pool, stream);
-    if (e != cudaSuccess) {
-      (void)cudaGetLastError();
-      return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: scratch for the slices of K: %s", cudaGetErrorString(e));
+    const size_t floats = PlanScratch(pl, mb, p->N);
+    if (caller.scratch != nullptr) {
+      if (floats > caller.scratch_floats) return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: %zu floats of scratch, %zu needed", caller.scratch_floats, floats);
+      a.scratch = caller.scratch;
+    } else {
+      // stream-ordered memory of the context's pool (an allocation node under capture)
+      const cudaError_t e = cudaMallocFromPoolAsync(&scratch, floats * sizeof(float), ctx->pool, stream);
+      if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return Fail(B200_RESOURCE_EXHAUSTED, "b200_qmm: scratch for the slices of K: %s", cudaGetErrorString(e));
+      }
+      a.scratch = static_cast<float*>(scratch);
     }
-    a.scratch = static_cast<float*>(scratch);
   }
   cudaError_t e;
   if (p->bits == 4 && p->nibble_order == 0) e = LaunchBatch<kInt4Seq, true>(mb, pl, map, a, max_smem, stream);

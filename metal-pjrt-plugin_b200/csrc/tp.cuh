@@ -58,6 +58,9 @@ struct QmmCaller {
   // dependents start: the product may request them while the kernel before it still runs.  Anyone else's weights may be
   // that kernel's output (kernels here let their dependents start before they store), so their product waits first.
   bool weights_settled = false;
+  // Scratch for products of 9 to 32 rows (QmmMidScratchFloats); null: pool memory of the call.
+  float* scratch = nullptr;
+  size_t scratch_floats = 0;
 };
 b200_status QmmRunEx(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p, const QmmCaller& caller);
 // Fills the fields above (push and consume sides) from a connected group; false when the exchange is not connected.

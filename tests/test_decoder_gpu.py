@@ -414,3 +414,64 @@ def test_step_refuses_bad_token_and_position(step_path):
             assert all(np.array_equal(x.view(np.uint16), y.view(np.uint16)) for x, y in zip(before, after))
         dec.close()
         ctx.close()
+
+
+def _tensors(cfg, batch):
+    import torch
+    p = pkg()
+    params, cache, tokens = inputs.config5(cfg, batch, 20, max_len=32)
+    dec = p.qwen3.Decoder(dev_params(params), {k: [dev(a) for a in v] for k, v in cache.items()}, cfg, max_batch=batch)
+    return p, dec, dev(tokens.astype(np.int32)), torch.tensor([20], dtype=torch.int32, device="cuda"), torch.empty((batch, cfg["vocab"]), device="cuda")
+
+
+@pytest.mark.parametrize("batch", [8, 9, 32])
+def test_a_step_allocates_nothing(batch, monkeypatch):
+    """The captured step holds no allocation node: the device's graph memory stays unused."""
+    import ctypes
+    import torch
+    monkeypatch.delenv("B200_DECODER_STREAM", raising=False)
+    cfg = inputs.decoder_config(layers=2, hidden=1024, heads=8, kv_heads=2, head_dim=128, inter=3072, vocab=2048)
+    p, dec, tok, pos, logits = _tensors(cfg, batch)
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.12")     # (torch's)
+    high, zero = ctypes.c_uint64(), ctypes.c_uint64(0)
+    used_high = 1                           # cudaGraphMemAttrUsedMemHigh
+    assert rt.cudaDeviceSetGraphMemAttribute(0, used_high, ctypes.byref(zero)) == 0
+    for _ in range(3):
+        dec.step(tok, pos, logits)
+    torch.cuda.synchronize()
+    assert rt.cudaDeviceGetGraphMemAttribute(0, used_high, ctypes.byref(high)) == 0 and high.value == 0
+    assert dec.graphs_built() == 1
+
+
+@pytest.mark.parametrize("batch", [3, 9, 32])
+def test_a_step_inside_the_callers_capture(batch, monkeypatch):
+    """A step that enqueues its kernels directly, captured with the sampling in the caller's own graph."""
+    import torch
+    monkeypatch.delenv("B200_DECODER_STREAM", raising=False)
+    monkeypatch.setenv("B200_DECODER_NO_GRAPH", "1")
+    cfg = inputs.decoder_config(layers=2, hidden=1024, heads=8, kv_heads=2, head_dim=128, inter=3072, vocab=2048)
+    p, dec, tok, pos, logits = _tensors(cfg, batch)
+    u = torch.full((batch,), 0.5, device="cuda")
+    dec.step(tok, pos, logits)
+    want, token = logits.clone(), p.qwen3.sample(logits, u, temperature=0.7, top_k=20)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dec.step(tok, pos, logits)
+        got = p.qwen3.sample(logits, u, temperature=0.7, top_k=20)
+    for _ in range(3):
+        logits.zero_()
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(logits, want) and torch.equal(got, token)
+
+
+@pytest.mark.parametrize("batch", [9, 17])
+def test_a_head_of_odd_width(batch, monkeypatch):
+    """More than 8 rows whose logits are not a multiple of eight: the head goes past the dense product and its widening pass."""
+    monkeypatch.delenv("B200_DECODER_STREAM", raising=False)
+    cfg = inputs.decoder_config(layers=1, hidden=512, heads=4, kv_heads=2, head_dim=128, inter=1024, vocab=1001)
+    for got, want in _run_decoder(cfg, batch, ctx=10, max_len=16)[0]:
+        _check_logits(got, want)
