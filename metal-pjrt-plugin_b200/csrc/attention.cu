@@ -11,7 +11,9 @@
 // latency per CTA).  Both products run on mma.sync with the query heads as the 8-wide operand and the cache bytes, as
 // loaded, as the 16-row one (positions for q.k, head dimensions for p.v): multiply-adds on the FMA pipes, with a shared
 // load for every eight of them, kept an SM busy twice as long as its share of the KV bytes takes.  The f32 probabilities
-// go in as three bf16 terms, which hold all of their 24 bits.  Decoder step (6 layers) at batch 32, position 2048:
+// go in as three bf16 terms, which hold all of their 24 bits, and every MMA of a leading term starts from zero, its sum being added in
+// f32: along a chain of accumulators the tensor core drops low bits (merged partials, D 128, position 777, against float64: FMA chains
+// 1.9e-7, accumulator chains 3.4e-7, as here 1.5e-7; no difference in time).  Decoder step (6 layers) at batch 32, position 2048:
 // 1636 -> 1264 us; batch 8, position 777: 661 -> 611; batch 1, position 2048: 380 -> 361.  (Longer runs of chunks per CTA,
 // prefetched, were slower than a CTA per chunk: 1697 -> 1754 us at batch 32.)  In the fused form the kernel also does what precedes
 // attention in the layer (qwen3.py:366-369): per-head RMSNorm and rotate-half
@@ -214,8 +216,11 @@ __global__ void __launch_bounds__(kThreads, 4) attn_partial_kernel(const AttnArg
 #pragma unroll
   for (int v = 0; v < KB; ++v) {
     const uint4 q = g < G ? *reinterpret_cast<const uint4*>(&qs[g < G ? g : 0][32 * v + 8 * t]) : make_uint4(0, 0, 0, 0);
-    mma_bf16_16816(c, kreg[0][v].x, kreg[1][v].x, kreg[0][v].y, kreg[1][v].y, q.x, q.y);
-    mma_bf16_16816(c, kreg[0][v].z, kreg[1][v].z, kreg[0][v].w, kreg[1][v].w, q.z, q.w);
+    float d[2][4];
+    mma_bf16_16816_z(d[0], kreg[0][v].x, kreg[1][v].x, kreg[0][v].y, kreg[1][v].y, q.x, q.y);
+    mma_bf16_16816_z(d[1], kreg[0][v].z, kreg[1][v].z, kreg[0][v].w, kreg[1][v].w, q.z, q.w);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[e] += d[0][e] + d[1][e];
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
@@ -281,12 +286,17 @@ __global__ void __launch_bounds__(kThreads, 4) attn_partial_kernel(const AttnArg
     uint32_t term[3][4];
     split3(pr, term);
 #pragma unroll
-    for (int k = 2; k >= 0; --k)   // the small terms first
+    for (int i = 0; i < DT; ++i) {
+      float d[2][4], small[4];
+      mma_bf16_16816_z(small, vreg[i][0][v].x, vreg[i][1][v].x, vreg[i][0][v].y, vreg[i][1][v].y, term[2][0], term[2][1]);
+      mma_bf16_16816(small, vreg[i][0][v].z, vreg[i][1][v].z, vreg[i][0][v].w, vreg[i][1][v].w, term[2][2], term[2][3]);
+      mma_bf16_16816(small, vreg[i][0][v].x, vreg[i][1][v].x, vreg[i][0][v].y, vreg[i][1][v].y, term[1][0], term[1][1]);
+      mma_bf16_16816(small, vreg[i][0][v].z, vreg[i][1][v].z, vreg[i][0][v].w, vreg[i][1][v].w, term[1][2], term[1][3]);
+      mma_bf16_16816_z(d[0], vreg[i][0][v].x, vreg[i][1][v].x, vreg[i][0][v].y, vreg[i][1][v].y, term[0][0], term[0][1]);
+      mma_bf16_16816_z(d[1], vreg[i][0][v].z, vreg[i][1][v].z, vreg[i][0][v].w, vreg[i][1][v].w, term[0][2], term[0][3]);
 #pragma unroll
-      for (int i = 0; i < DT; ++i) {
-        mma_bf16_16816(o[i], vreg[i][0][v].x, vreg[i][1][v].x, vreg[i][0][v].y, vreg[i][1][v].y, term[k][0], term[k][1]);
-        mma_bf16_16816(o[i], vreg[i][0][v].z, vreg[i][1][v].z, vreg[i][0][v].w, vreg[i][1][v].w, term[k][2], term[k][3]);
-      }
+      for (int e = 0; e < 4; ++e) o[i][e] += (small[e] + d[0][e]) + d[1][e];
+    }
   }
   // An infinite value meets the zero terms of its probability as NaN: such sums are formed again, term by term.
 #pragma unroll
