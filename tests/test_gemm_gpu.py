@@ -283,3 +283,44 @@ def test_matmul_takes_a_trailing_dimension_of_one():
     p = pkg()
     a, b = torch.randn((5, 64), device="cuda"), torch.randn((64, 33), device="cuda")
     assert torch.equal(p.blas.matmul(a, b[:, :, None]), p.blas.matmul(a, b))
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("act", [2, 3])
+def test_activation_of_every_input(act, dt):
+    """The epilogue's SiLU and GELU of every 16-bit input, from a product with one column of ones: one rounding of the float64 value, plus
+    2^-21 for the f32 arithmetic (GELU: of its exponent z too, 4 roundings times |z|).  A reciprocal flushed to zero, or an exponent
+    whose rounding is not made good, shows for large negative inputs."""
+    import torch
+    p = pkg()
+    t = torch.bfloat16 if dt == "bf16" else torch.float16
+    v = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(t)
+    x = torch.zeros((65536, 64), dtype=t, device="cuda")
+    one = torch.zeros((64, 64), dtype=t, device="cuda")
+    ok = torch.isfinite(v) & (v.abs() < 1e4)
+    x[:, 0] = torch.where(ok, v, torch.zeros_like(v))
+    one[0] = 1
+    got = p.blas.matmul(x, one, None, act)
+    assert torch.equal(got, got[:, :1].expand(-1, 64))
+    a, got = x[:, 0].double(), got[:, 0].double()
+    z = a if act == 3 else 2 * 0.7978845608028654 * (a + 0.044715 * a ** 3)
+    want = a / (1 + torch.exp(-z))
+    smallest = 2.0 ** -134 if dt == "bf16" else 2.0 ** -25      # half a step of the subnormals
+    # half a step just above a power of two: 2^-8 of the value with 8 significant bits, 2^-11 with 11
+    rel = (2.0 ** -8 if dt == "bf16" else 2.0 ** -11) + 2.0 ** -21 + (z.abs() * 2.0 ** -22 if act == 2 else 0.0)
+    err = (got - want).abs() - (want.abs() * rel + smallest)
+    near = z > -88.7                     # beyond, exp(-z) is not an f32 number and the result is zero
+    assert bool((err[near] <= 0).all()), (float(err[near].max()), float(a[near][err[near].argmax()]))
+    assert bool((got[~near].abs() <= want[~near].abs() + smallest).all())
+
+
+@pytest.mark.parametrize("act", [1, 2, 3])
+def test_activation_of_infinities_and_nan(act):
+    import torch
+    p = pkg()
+    x = torch.zeros((200, 64), dtype=torch.bfloat16, device="cuda")
+    x[0, 0], x[1, 0], x[2, 0], x[3, 0], x[4, 0] = float("inf"), float("nan"), 3e38, -3e38, -200.0
+    one = torch.zeros((64, 64), dtype=torch.bfloat16, device="cuda")
+    one[0] = 1
+    got = p.blas.matmul(x, one, None, act)[:, 0].float().cpu()
+    assert got[0] == float("inf") and got[1].isnan() and got[2] == x[2, 0].float().cpu() and got[3] == 0 and got[4] == 0
