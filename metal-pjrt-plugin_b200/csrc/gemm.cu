@@ -338,8 +338,14 @@ b200_status RunTcgen05Aligned(b200_context* ctx, cudaStream_t stream, const b200
   return s;
 }
 
+// f32 results show the low bits that the tensor core's accumulator drops (bf16 operands, k = 1625, against float64: 1.6e-6, the SIMT
+// kernel 3.4e-7), results of 16 bits do not.  One aligned product takes the tensor core for either; batches and copied operands,
+// where the SIMT kernel is the alternative in earnest, only for 16-bit results (or where the caller asks for that route).
+bool KeepsPrecision(const b200_gemm_params* p) { return p->c.dtype != B200_F32; }
+
 // Worth an aligned copy: the SIMT kernel runs at about 20 TFLOP/s, the copies cost a few microseconds each.
 bool WorthAligning(const b200_gemm_params* p, const b200_epilogue* epi) {
+  if (!KeepsPrecision(p)) return false;
   b200_gemm_params q = *p;
   for (b200_operand* x : {&q.a, &q.b})
     if (!TmaReadable(*x, p->batch)) x->ptr = nullptr, x->ld = 8, x->batch_stride = 0;
@@ -401,7 +407,7 @@ int Route(const b200_gemm_params* p, const b200_epilogue* epi, int forced) {
   if (forced == B200_ROUTE_TCGEN05 && tc) return B200_ROUTE_TCGEN05;
   // measured on 4096 x 4096 weights: 9 vs 13 us at 1 row, 12 vs 14 at 8, 20 vs 13 at 16, 33 vs 16 at 32
   if (few && (std::min(p->m, p->n) <= 8 || !tc)) return B200_ROUTE_FEWROW;
-  if (tc || WorthAligning(p, epi)) return B200_ROUTE_TCGEN05;
+  if ((tc && (p->batch == 1 || KeepsPrecision(p))) || WorthAligning(p, epi)) return B200_ROUTE_TCGEN05;
   return B200_ROUTE_SIMT;
 }
 

@@ -324,3 +324,20 @@ def test_activation_of_infinities_and_nan(act):
     one[0] = 1
     got = p.blas.matmul(x, one, None, act)[:, 0].float().cpu()
     assert got[0] == float("inf") and got[1].isnan() and got[2] == x[2, 0].float().cpu() and got[3] == 0 and got[4] == 0
+
+
+@pytest.mark.parametrize("dt,batch,m,n,k", [("bf16", 1, 777, 1001, 1625), ("f16", 1, 1625, 1625, 333), ("bf16", 3, 512, 512, 2048), ("f16", 5, 777, 777, 128)])
+def test_f32_results_of_16_bit_operands_keep_f32_sums(dt, batch, m, n, k):
+    """Batches and unaligned rows: a sum of k terms in f32, added in blocks, is within sqrt(k) 2^-25 of float64 in the 2-norm; the tensor core's
+    accumulator is at four times that."""
+    import torch
+    p = pkg()
+    t = torch.bfloat16 if dt == "bf16" else torch.float16
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = torch.randn((batch, m, k), generator=g, device="cuda").to(t), torch.randn((batch, k, n), generator=g, device="cuda").to(t)
+    d = torch.empty((batch, m, n), device="cuda")
+    B = p.blas
+    B.run_steel_gemm(B.GemmParams(m, n, k, B.Operand(a, k, m * k), B.Operand(b, n, k * n), B.Operand(d, n, m * n), batch))
+    want = a.double() @ b.double()
+    err = float((d.double() - want).norm() / want.norm())
+    assert err <= k ** 0.5 * 2.0 ** -25, err
