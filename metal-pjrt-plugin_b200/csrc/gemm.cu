@@ -38,6 +38,7 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
 
 namespace {
 
+constexpr size_t kSmemPerSm = 228 * 1024;   // 1 KB of it is taken by each CTA beside what it asks for
 constexpr int64_t kMaxInt = INT32_MAX;
 constexpr int64_t kMaxLd = INT32_MAX / 256;  // steel_gemm.cc:153
 
@@ -56,6 +57,11 @@ struct SimtArgs {
   int split;           // CTAs of a cluster along K
 };
 
+__device__ __forceinline__ void add_pair(float2& d, const float2& a) {
+  asm("{\n\t.reg .b64 x, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 z, {%0, %1};\n\tadd.rn.f32x2 z, z, x;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "+f"(d.x), "+f"(d.y)
+      : "f"(a.x), "f"(a.y));
+}
 // d += {a, a} * {b0, b1}: two IEEE multiply-adds per lane in one instruction, so that the FMA pipes are kept busy
 // with half of the issue slots and the rest go to loads.
 __device__ __forceinline__ void fma_pair(float2& d, float a, const float2& b) {
@@ -68,23 +74,29 @@ __device__ __forceinline__ void fma_pair(float2& d, float a, const float2& b) {
 
 // One shape of the tile kernel: a BM x BN tile by KG groups of threads, TM x TN values a thread; a group takes its own
 // part of every BK-deep step.
-template <int BM_, int BN_, int TM_, int TN_, int KG_, int BK_>
+template <int BM_, int BN_, int TM_, int TN_, int KG_, int BK_, int RESIDENT_>
 struct Tile {
+  static constexpr int kResident = RESIDENT_;   // CTAs per SM that registers are kept for
+  static constexpr bool kDirect = KG_ == 1 && BM_ == 64;   // results go from registers to memory; no split of K
   static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KG = KG_, BK = BK_;
   static constexpr int kGroup = (BM / TM) * (BN / TN);
   static constexpr int kThreads = kGroup * KG;
   static constexpr int kPitchA = BM + 4, kPitchB = BN + 4;   // floats; keeps 16-byte reads aligned
   static constexpr int kBuffer = BK * (kPitchA + kPitchB);   // floats of one of the two steps held
-  static constexpr size_t kSmem = sizeof(float) * (2 * kBuffer > KG * BM * BN ? 2 * kBuffer : KG * BM * BN);
+  static constexpr size_t kSmem = sizeof(float) * (kDirect || 2 * kBuffer > KG * BM * BN ? 2 * kBuffer : KG * BM * BN);
   static constexpr int kLoadsA = BM * BK / kThreads, kLoadsB = BN * BK / kThreads;
   static_assert(BM * BK % kThreads == 0 && BN * BK % kThreads == 0 && kThreads % BK == 0 && kThreads % BM == 0 && kThreads % BN == 0, "");
 };
 // Large products: 8 x 8 values a thread (a step of k costs 4 shared loads of 16 bytes for 32 paired multiply-adds).
-using Large = Tile<128, 128, 8, 8, 1, 16>;
+using Large = Tile<128, 128, 8, 8, 1, 16, 2>;
 // Products whose 128 x 128 tiles leave SMs idle: two groups of four warps on a 64 x 64 tile.
-using Medium = Tile<64, 64, 4, 8, 2, 32>;
+using Medium = Tile<64, 64, 4, 8, 2, 32, 1>;
 // Few rows: eight groups of two warps, each with its own part of k.
-using Few = Tile<16, 64, 4, 4, 8, 64>;
+using Few = Tile<16, 64, 4, 4, 8, 64, 1>;
+// Many tiles of a short K: what a tile costs beside its multiply-adds (the first loads, the last step, the stores) is hidden by
+// other CTAs of the same SM, not by more work per thread.  Sums of 32 values are added up, as finely as the medium tile's two groups
+// have it.
+using Short = Tile<64, 64, 4, 4, 1, 16, 4>;
 
 // One thread's share of a step of an operand: `kLoads` values, along the operand's contiguous dimension first.
 // OUTER: rows of op(A) or columns of op(B); BYK: k is the contiguous dimension.
@@ -121,7 +133,7 @@ struct Loader {
 // f32 512 x 1024 x 1024: 81 us with 4 x 4 values a thread and unpaired multiply-adds -> 45; 2048 x 2048 x 1024 runs at
 // 35 TFLOP/s.
 template <typename TIn, typename TOut, typename T>
-__global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_kernel(const SimtArgs p) {
+__global__ void __launch_bounds__(T::kThreads, T::kResident) gemm_simt_kernel(const SimtArgs p) {
   constexpr int BM = T::BM, BN = T::BN, TM = T::TM, TN = T::TN, BK = T::BK;
   extern __shared__ __align__(16) float smem_f[];
   pdl_wait();
@@ -157,6 +169,14 @@ __global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_ker
 #pragma unroll
     for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
 
+  float2 sums[T::kDirect ? TM : 1][TN / 2];   // finished sums of 32 values of k
+  if constexpr (T::kDirect) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) sums[i][j] = make_float2(0.0f, 0.0f);
+  }
+
   if (s0 < s1) {
     la.load(p.k - s0 * BK, va);
     lb.load(p.k - s0 * BK, vb);
@@ -190,10 +210,42 @@ __global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_ker
           }
       }
     }
+    if constexpr (T::kDirect) {
+      if ((s & 1) != 0 || s + 1 == s1) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN / 2; ++j) {
+            add_pair(sums[i][j], acc[i][j]);
+            acc[i][j] = make_float2(0.0f, 0.0f);
+          }
+      }
+    }
     if (s + 1 < s1) put(smem_f + ((s + 1 - s0) & 1) * T::kBuffer);   // (last read in the step before: the barrier below)
     __syncthreads();
   }
 
+  TOut* D = static_cast<TOut*>(p.d) + batch * p.sd;
+  TOut* AUX = p.aux ? static_cast<TOut*>(p.aux) + batch * p.sd : nullptr;
+  auto finish = [&](int gi, int gj, float sum) {
+    const int64_t o = static_cast<int64_t>(gi) * p.ldd + gj;
+    float v = p.alpha * sum;
+    if (p.beta != 0.0f) v += p.beta * load_as_f32<TOut>(D + o);
+    if (p.bias != nullptr) v += load_as_f32<TOut>(static_cast<const TOut*>(p.bias) + gj);
+    if (AUX != nullptr) AUX[o] = store_from_f32<TOut>(v);
+    D[o] = store_from_f32<TOut>(apply_act(p.act, v));
+  };
+  if constexpr (T::kDirect) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int gi = m0 + ty * 4 + i;
+      if (gi >= p.m) continue;
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+        if (n0 + tx * 4 + j < p.n) finish(gi, n0 + tx * 4 + j, (j & 1) ? sums[i][j / 2].y : sums[i][j / 2].x);
+    }
+    return;
+  }
   // ---- the groups' tiles -> shared memory [group][BM][BN]
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -206,8 +258,6 @@ __global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_ker
   cg::cluster_group cl = cg::this_cluster();
   if (p.split > 1) cl.sync();
   else __syncthreads();
-  TOut* D = static_cast<TOut*>(p.d) + batch * p.sd;
-  TOut* AUX = p.aux ? static_cast<TOut*>(p.aux) + batch * p.sd : nullptr;
   for (int e = rank * T::kThreads + tid; e < BM * BN; e += p.split * T::kThreads) {
     const int gi = m0 + e / BN, gj = n0 + e % BN;
     if (gi >= p.m || gj >= p.n) continue;
@@ -217,55 +267,64 @@ __global__ void __launch_bounds__(T::kThreads, T::KG == 1 ? 2 : 1) gemm_simt_ker
 #pragma unroll
       for (int g = 0; g < T::KG; ++g) sum += t[g * BM * BN + e];
     }
-    const int64_t o = static_cast<int64_t>(gi) * p.ldd + gj;
-    float v = p.alpha * sum;
-    if (p.beta != 0.0f) v += p.beta * load_as_f32<TOut>(D + o);
-    if (p.bias != nullptr) v += load_as_f32<TOut>(static_cast<const TOut*>(p.bias) + gj);
-    if (AUX != nullptr) AUX[o] = store_from_f32<TOut>(v);
-    D[o] = store_from_f32<TOut>(apply_act(p.act, v));
+    finish(gi, gj, sum);
   }
   if (p.split > 1) cl.sync();   // the peers may still be reading this CTA's tile
 }
 
 template <typename TIn, typename TOut, typename T>
-cudaError_t LaunchTile(const SimtArgs& a, int64_t batch, cudaStream_t stream) {
+cudaError_t LaunchTile(const SimtArgs& a, int64_t batch, cudaStream_t stream, size_t smem = T::kSmem) {
   auto kernel = gemm_simt_kernel<TIn, TOut, T>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T::kSmem));
+  smem = std::max(smem, T::kSmem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   LaunchCfg lc;
   lc.grid = dim3(static_cast<unsigned>(CeilDiv(a.n, T::BN) * a.split), static_cast<unsigned>(CeilDiv(a.m, T::BM)),
                  static_cast<unsigned>(batch));
   lc.block = dim3(T::kThreads);
-  lc.smem = T::kSmem;
+  lc.smem = smem;
   lc.stream = stream;
   lc.pdl = true;
   lc.cluster_x = a.split;
   return Launch(lc, kernel, a);
 }
 
-// The tile by its cost in multiply-adds on the busiest SM, weighted by how well each shape keeps the pipes busy; then,
-// where tiles are too few for the SMs, a split of K.
+// The tile by its time, in microseconds fitted to 148 SMs (f32, 16 sets of sizes, K from 16 to 4096): the busiest SM takes `n` tiles,
+// each a fixed part and a part per value of k; short tiles run up to four at a time.  Where few tiles leave SMs
+// idle, a cluster splits K.  Measured with the short tile and with the best of the others (us): 32 x 777 x 777 x 128 202 / 253, 32 x 512 x
+// 512 x 64 49 / 71, 512 x 64 x 64 x 64 17 / 30, 100000 x 8 x 64 39 / 81; and where it loses: 1024 x 1024 x 1024 92 / 89 (medium), 4096 x 4096 x
+// 512 540 / 432 (large), 300 x 200 x 256 19 / 7 (few).
 template <typename TIn, typename TOut>
 cudaError_t LaunchSimt(SimtArgs a, int64_t batch, int sm_count, cudaStream_t stream) {
   auto tiles = [&](int bm, int bn) { return CeilDiv(a.m, bm) * CeilDiv(a.n, bn) * batch; };
-  auto cost = [&](int bm, int bn, double weight) { return static_cast<double>(CeilDiv(tiles(bm, bn), sm_count)) * bm * bn * weight; };
   auto split = [&](int64_t count) {
     int s = 1;
     while (s < 8 && count * s * 2 <= sm_count && a.k / (2 * s) >= 256) s *= 2;
     return s;
   };
-  const bool tall_ok = CeilDiv(a.m, 16) <= 65535;
-  const double large = cost(128, 128, 1.0), medium = cost(64, 64, 1.15), few = tall_ok ? cost(16, 64, 2.0) : 1e30;
-  if (few < medium && few < large) {
-    a.split = split(tiles(16, 64));
-    return LaunchTile<TIn, TOut, Few>(a, batch, stream);
+  auto turns = [&](int bm, int bn) { return static_cast<double>(CeilDiv(tiles(bm, bn), sm_count)); };
+  const int s_few = split(tiles(16, 64)), s_medium = split(tiles(64, 64));
+  const double k = a.k, n_large = turns(128, 128), n_64 = turns(64, 64);
+  // (of clusters of eight, of which a GPC takes whole ones only, about twelve are resident at once)
+  auto waves = [&](int s, int64_t count) { return s == 8 && count > 12 ? 2.0 : 1.0; };
+  const double few = CeilDiv(a.m, 16) > 65535 ? 1e30 : turns(16, 64) * (0.016 * k / s_few + 1.8) * waves(s_few, tiles(16, 64)) + (s_few > 1 ? 3.0 : 1.5);
+  const double medium = n_64 * (0.0385 * k / s_medium + 4.5) * waves(s_medium, tiles(64, 64)) + (s_medium > 1 ? 3.0 : 1.5);
+  const double large = n_large == 1 ? 0.1225 * k + 20.0 : n_large * (0.1 * k + 11.3) + 2.0;
+  const double short_k = n_64 == 1 ? 0.055 * k + 5.5 : (n_64 == 2 ? 0.085 * k + 5.5 : (n_64 == 3 ? 0.118 * k + 6.5 : n_64 * (0.037 * k + 1.05) + 2.0));
+  const double best = std::min({few, medium, large, short_k});
+  a.split = 1;
+  if (best == short_k) {
+    // Up to four tiles per SM: shared memory for just that many, or some SMs get four and others one.
+    const size_t share = n_64 <= 4 ? kSmemPerSm / static_cast<size_t>(n_64) - 1024 : 0;
+    return LaunchTile<TIn, TOut, Short>(a, batch, stream, share);
   }
-  if (medium < large) {
-    a.split = split(tiles(64, 64));
+  if (best == large) return LaunchTile<TIn, TOut, Large>(a, batch, stream);
+  if (best == medium) {
+    a.split = s_medium;
     return LaunchTile<TIn, TOut, Medium>(a, batch, stream);
   }
-  a.split = 1;
-  return LaunchTile<TIn, TOut, Large>(a, batch, stream);
+  a.split = s_few;
+  return LaunchTile<TIn, TOut, Few>(a, batch, stream);
 }
 
 // Copies rows of `cols` 16-bit elements that start anywhere into rows of `dst_words` 32-bit words.  Bound by memory:

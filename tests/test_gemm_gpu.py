@@ -341,3 +341,14 @@ def test_f32_results_of_16_bit_operands_keep_f32_sums(dt, batch, m, n, k):
     want = a.double() @ b.double()
     err = float((d.double() - want).norm() / want.norm())
     assert err <= k ** 0.5 * 2.0 ** -25, err
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(63, 65, 1, 75), (65, 127, 33, 40), (777, 300, 47, 4), (1000, 513, 129, 2), (4100, 7, 100, 3), (640, 640, 64, 2),
+                                         (1280, 641, 80, 1), (64, 64, 15, 160)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+def test_simt_short_tile(m, n, k, batch, ta, tb):
+    """The general kernel's tile for many products of a short K: one to six tiles per SM, ragged edges, steps that end early."""
+    p = pkg()
+    run_case(m, n, k, batch=batch, dt_in="f32", ta=ta, tb=tb, pad=1, alpha=0.5, beta=1.5, bias=True, act=2, aux=True, route=p._lib.ROUTE_SIMT)
+    run_case(m, n, k, batch=batch, ta=ta, tb=tb, dt_in="f16", dt_out="f32", broadcast_b=batch > 1, route=p._lib.ROUTE_SIMT)
+
