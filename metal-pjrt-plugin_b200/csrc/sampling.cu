@@ -50,18 +50,21 @@ struct SampleArgs {
   float top_p;
 };
 
-struct Shared {
+// What both kernels use.
+struct Common {
   unsigned long long cand[kMaxCand];
-  unsigned maxima[kMaxCluster * kT];   // keys of all threads' maxima, of all CTAs
-  float parts[kT];                     // sums of all chunks; later the cumulative probabilities
-  float cta_max[kMaxCluster];
-  int cta_arg[kMaxCluster];
+  float parts[kT];                     // cluster: sums of all chunks; later the cumulative probabilities
   float s_val[kT / 32];
   int s_idx[kT / 32];
   float warp_tot[kT / 32];
-  unsigned warp_cnt[2][kT / 32];
   unsigned hist[256];
   unsigned prefix, krem, count, choice;
+};
+struct Shared : Common {
+  unsigned maxima[kMaxCluster * kT];   // keys of all threads' maxima, of all CTAs
+  float cta_max[kMaxCluster];
+  int cta_arg[kMaxCluster];
+  unsigned warp_cnt[2][kT / 32];
 };
 constexpr size_t kHeader = (sizeof(Shared) + 15) / 16 * 16;
 
@@ -69,6 +72,19 @@ constexpr size_t kHeader = (sizeof(Shared) + 15) / 16 * 16;
 __device__ __forceinline__ uint32_t fkey(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// The largest value of a warp's lanes and its lowest index, in every lane.
+__device__ __forceinline__ void best_of_warp(float& v, int& i) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+    if (ov > v || (ov == v && oi < i)) {
+      v = ov;
+      i = oi;
+    }
+  }
 }
 
 // Inclusive scan over the block's kT threads (deterministic: warp scans, then the warp totals).
@@ -99,7 +115,7 @@ __device__ __forceinline__ float block_scan(float v, float* warp_tot, float* tot
 
 // The exact top k of a row by one CTA: the k-th largest key by radix selection (four passes of eight bits), then
 // every key above it and the lowest indices of its equals, into cand[0 .. k).
-__device__ __noinline__ void select_exact(Shared& sh, const float* x, int V, int k) {
+__device__ __noinline__ void select_exact(Common& sh, const float* x, int V, int k) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     sh.prefix = 0;
@@ -185,6 +201,68 @@ __device__ __forceinline__ void read_share(const float* x, int lo, int hi, int c
   }
 }
 
+// Sorts the gathered candidates and draws among the first k: nucleus, then the inverse CDF.  sh.choice is 0xffffffff.
+__device__ __forceinline__ void draw_sorted(Common& sh, const SampleArgs& a, const float* x, float gmax, float u, unsigned n_cand, int row) {
+  const int tid = threadIdx.x, k = a.top_k;
+  // ---- bitonic sort, descending (value, then lower index first)
+  unsigned slots = 32;
+  while (slots < n_cand) slots <<= 1;
+  for (unsigned i = n_cand + tid; i < slots; i += kT) sh.cand[i] = 0ull;
+  __syncthreads();
+  for (unsigned size = 2; size <= slots; size <<= 1) {
+    for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
+      if (static_cast<unsigned>(tid) < slots / 2) {
+        const unsigned i = 2 * tid - (tid & (stride - 1)), j = i + stride;
+        const unsigned long long p = sh.cand[i], q = sh.cand[j];
+        if ((p < q) == ((i & size) == 0)) {
+          sh.cand[i] = q;
+          sh.cand[j] = p;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // ---- probabilities of the sorted candidates, nucleus, draw
+  float pj = 0.0f;
+  int idx = 0;
+  if (tid < k) {
+    idx = static_cast<int>(0xffffffffu - static_cast<unsigned>(sh.cand[tid] & 0xffffffffull));
+    pj = expf((x[idx] - gmax) * a.inv_temperature);
+  }
+  float total;
+  const float cum = block_scan(pj, sh.warp_tot, &total);
+  if (tid < kMaxTopK) sh.parts[tid] = cum;
+  // kept: before < top_p * total (the first candidate always is)
+  const bool kept = tid < k && (tid == 0 || (cum - pj) < a.top_p * total);
+  float kcount;
+  block_scan(kept ? 1.0f : 0.0f, sh.warp_tot, &kcount);
+  const int kk = max(1, static_cast<int>(kcount));
+  const float kept_total = sh.parts[kk - 1];
+  const float target = u * kept_total;
+  // The first candidate whose cumulative probability exceeds the target.  (Not "the one whose interval holds it": intervals formed
+  // from the scan overlap, or leave gaps, in their last bit.)
+  if (tid < kk && pj > 0.0f && target < cum) atomicMin(&sh.choice, static_cast<unsigned>(tid));
+  __syncthreads();
+  const unsigned at = sh.choice == 0xffffffffu ? static_cast<unsigned>(kk - 1) : sh.choice;   // none: u * total rounded up to the total
+  if (static_cast<unsigned>(tid) == at) a.out[row] = idx;
+}
+
+// The draw inside a chunk [i0, i1) of the row whose exponentials come from `e`: the first one whose cumulative sum exceeds the target, the last
+// one that is not zero where rounding leaves none.
+template <typename F>
+__device__ __forceinline__ int walk_chunk(int i0, int i1, float before, float target, F e) {
+  float c = before;
+  int pick = i0;
+  for (int i = i0; i < i1; ++i) {
+    const float v = e(i);
+    if (!(v > 0.0f)) continue;
+    pick = i;
+    c += v;
+    if (target < c) break;
+  }
+  return pick;
+}
+
 // grid = (cluster, rows)
 __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -209,15 +287,7 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
   if (a.stash && a.inv_temperature != 0.0f) read_share<true>(x, lo, hi, chunk, stash, bv, bi);
   else read_share<false>(x, lo, hi, chunk, stash, bv, bi);
   const unsigned mykey = lo + tid < hi ? fkey(bv) : 0u;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ov > bv || (ov == bv && oi < bi)) {
-      bv = ov;
-      bi = oi;
-    }
-  }
+  best_of_warp(bv, bi);
   if (lane == 0) {
     sh.s_val[warp] = bv;
     sh.s_idx[warp] = bi;
@@ -231,15 +301,7 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
   if (warp == 0) {
     float v = sh.s_val[lane];
     int i = sh.s_idx[lane];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-      if (ov > v || (ov == v && oi < i)) {
-        v = ov;
-        i = oi;
-      }
-    }
+    best_of_warp(v, i);
     if (lane < C) {
       Shared* peer = cl.map_shared_rank(&sh, lane);
       peer->cta_max[rank] = v;
@@ -286,9 +348,9 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
     const float part = sh.parts[tid];
     float total;
     const float incl = block_scan(part, sh.warp_tot, &total);
-    const float target = u * total, before = incl - part;
-    // (the differences of the scan may overlap in the last bit: the first chunk that holds the draw counts)
-    if (part > 0.0f && before <= target && target < incl) atomicMin(&sh.choice, static_cast<unsigned>(tid));
+    const float target = u * total;
+    // the first chunk that reaches beyond the target (the scan's differences overlap, or leave gaps, in their last bit)
+    if (part > 0.0f && target < incl) atomicMin(&sh.choice, static_cast<unsigned>(tid));
     __syncthreads();
     const unsigned owner = sh.choice;
     if (owner == 0xffffffffu) {
@@ -296,16 +358,7 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
     } else if (owner == static_cast<unsigned>(tid) && tid / cpc == rank) {
       const int i0 = min(tid * chunk, V), i1 = min(i0 + chunk, V);
       const float* e = stash + (tid - rank * cpc) * pitch;
-      float c = before;
-      int pick = i1 - 1;
-      for (int i = i0; i < i1; ++i) {
-        c += a.stash ? e[i - i0] : expf((x[i] - gmax) * a.inv_temperature);
-        if (target < c) {
-          pick = i;
-          break;
-        }
-      }
-      a.out[blockIdx.y] = pick;
+      a.out[blockIdx.y] = walk_chunk(i0, i1, incl - part, target, [&](int i) { return a.stash ? e[i - i0] : expf((x[i] - gmax) * a.inv_temperature); });
     }
     return;
   }
@@ -373,46 +426,7 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
     select_exact(sh, x, V, k);
     n_cand = static_cast<unsigned>(k);
   }
-  // ---- bitonic sort, descending (value, then lower index first)
-  unsigned slots = 32;
-  while (slots < n_cand) slots <<= 1;
-  for (unsigned i = n_cand + tid; i < slots; i += kT) sh.cand[i] = 0ull;
-  __syncthreads();
-  for (unsigned size = 2; size <= slots; size <<= 1) {
-    for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
-      if (static_cast<unsigned>(tid) < slots / 2) {
-        const unsigned i = 2 * tid - (tid & (stride - 1)), j = i + stride;
-        const unsigned long long p = sh.cand[i], q = sh.cand[j];
-        if ((p < q) == ((i & size) == 0)) {
-          sh.cand[i] = q;
-          sh.cand[j] = p;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // ---- probabilities of the sorted candidates, nucleus, draw
-  float pj = 0.0f;
-  int idx = 0;
-  if (tid < k) {
-    idx = static_cast<int>(0xffffffffu - static_cast<unsigned>(sh.cand[tid] & 0xffffffffull));
-    pj = expf((x[idx] - gmax) * a.inv_temperature);
-  }
-  float total;
-  const float cum = block_scan(pj, sh.warp_tot, &total);
-  if (tid < kMaxTopK) sh.parts[tid] = cum;
-  // kept: before < top_p * total (the first candidate always is)
-  const bool kept = tid < k && (tid == 0 || (cum - pj) < a.top_p * total);
-  float kcount;
-  block_scan(kept ? 1.0f : 0.0f, sh.warp_tot, &kcount);
-  const int kk = max(1, static_cast<int>(kcount));
-  const float kept_total = sh.parts[kk - 1];
-  const float target = u * kept_total;
-  if (tid < kk && (cum - pj) <= target && target < cum) sh.choice = static_cast<unsigned>(idx);
-  __syncthreads();
-  if (tid == kk - 1 && sh.choice == 0xffffffffu) sh.choice = static_cast<unsigned>(idx);   // u * total rounded up to the total
-  __syncthreads();
-  if (tid == 0) a.out[blockIdx.y] = static_cast<int>(sh.choice);
+  draw_sorted(sh, a, x, gmax, u, n_cand, blockIdx.y);
 }
 
 }  // namespace
@@ -449,18 +463,19 @@ b200_status b200_sample(b200_context* ctx, b200_stream stream, const float* logi
   // One wave of CTAs where that can be (a CTA's share and tables leave room for one per SM), and at least as many per
   // row as it takes for their shares to fit shared memory.
   a.chunk = static_cast<int>(CeilDiv(vocab, kT));
+  LaunchCfg lc;
+  lc.stream = stream;
+  lc.block = dim3(kT);
+  lc.pdl = true;
+  cudaError_t e;
   const bool fits4 = kHeader + static_cast<size_t>(kT / 4) * (a.chunk + 1) * sizeof(float) <= static_cast<size_t>(ctx->max_smem_optin);
   const int cluster = batch * 8 <= ctx->sm_count || !fits4 ? 8 : 4;
   const size_t share = static_cast<size_t>(kT / cluster) * (a.chunk + 1) * sizeof(float);
   a.stash = a.inv_temperature != 0.0f && kHeader + share <= static_cast<size_t>(ctx->max_smem_optin);
-  LaunchCfg lc;
-  lc.stream = stream;
   lc.grid = dim3(cluster, static_cast<unsigned>(batch));
-  lc.block = dim3(kT);
   lc.cluster_x = cluster;
-  lc.pdl = true;
   lc.smem = kHeader + (a.stash ? share : 0);
-  cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
+  e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem_optin);
   if (e == cudaSuccess) e = Launch(lc, sample_kernel, a);
   if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_sample launch: %s", cudaGetErrorString(e)));
   return EndLaunch(ctx, "b200_sample");

@@ -115,3 +115,44 @@ def test_numbers_of_any_type():
     want = _run(pkg(), logits, u, temperature=0.75, top_k=20, top_p=0.5)
     got = _run(pkg(), logits, u, temperature=np.float32(0.75), top_k=20.0, top_p=torch.tensor(0.5))
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [24, 4096])
+@pytest.mark.parametrize("kw", [dict(), dict(top_k=100), dict(top_k=1000, top_p=0.9)])
+def test_the_draw_is_monotone_in_the_uniform_number(rows, kw):
+    """An inverse CDF: of rows with the same logits, a larger number never draws an earlier candidate.  The numbers lie within 4 steps of f32 around
+    the edges between candidates (or chunks), where sums formed in different orders overlap and leave gaps."""
+    import torch
+    p = pkg()
+    rng = np.random.default_rng(3)
+    V, T = 2050, 0.7
+    logits = (rng.standard_normal(V) * 2).astype(np.float32)
+    order = np.argsort(-logits, kind="stable")[:kw["top_k"]] if kw else np.arange(V)
+    pr = np.exp((logits[order].astype(np.float64) - logits.max()) / T)
+    if "top_p" in kw:
+        pr = pr[:np.searchsorted(np.cumsum(pr), kw["top_p"] * pr.sum()) + 1]
+    edges = np.cumsum(pr)[:-1] / pr.sum()
+    u = np.sort(np.concatenate([np.float32(edges) + np.float32(2.0 ** -24) * i for i in range(-4, 5)])).astype(np.float32)
+    u = u[(u > 0) & (u < 1)]
+    place = np.full(V, -1)
+    place[order] = np.arange(len(order))
+    got = []
+    for i in range(0, len(u), rows):
+        part = u[i:i + rows]
+        ld = dev(logits)[None].expand(len(part), V).contiguous()
+        got.append(host(p.qwen3.sample(ld, dev(part), temperature=T, **kw)))
+    at = place[np.concatenate(got)]
+    assert (at >= 0).all() and (np.diff(at) >= 0).all(), np.flatnonzero(np.diff(at) < 0)[:10]
+
+
+def test_no_draw_of_an_impossible_token():
+    """Tokens masked with -inf have probability zero: not drawn whatever the number, the largest included."""
+    rng = np.random.default_rng(4)
+    for V in (1000, 50257):
+        logits = rng.standard_normal((64, V)).astype(np.float32)
+        logits[:, rng.permutation(V)[:V - 30]] = -np.inf
+        u = np.concatenate([rng.random(60), [0.0, 1 - 2.0 ** -24, 1 - 2.0 ** -23, 0.5]]).astype(np.float32)
+        for B in (64, 20):
+            for kw in (dict(), dict(top_k=25)):
+                got = _run(pkg(), logits[:B], u[64 - B:], temperature=0.9, **kw)
+                assert np.isfinite(logits[np.arange(B), got]).all()
