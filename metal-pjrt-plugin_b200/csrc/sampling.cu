@@ -13,7 +13,7 @@
 //
 // Bound by latency: one pass over the logits is 3 us of HBM for 32 rows of 151936, and one CTA per row
 // (which re-read its row from L2 six to ten times and met on single histogram counters) took 158 us for that.
-// A cluster of CTAs takes a row.  Each reads its share once into shared memory, where all later passes run;
+// A cluster of CTAs takes a row (many or short rows: one CTA each, see RowPerCta).  Each reads its share once into shared memory, where all later passes run;
 // the CTAs exchange maxima, thresholds and candidates by stores into each other's shared memory.
 //   top-k   every thread's maximum is one of kT x cluster groups, so the k-th largest maximum is a lower bound
 //           of the k-th largest logit, and hardly more than k logits reach it: those are gathered in the first
@@ -115,7 +115,7 @@ __device__ __forceinline__ float block_scan(float v, float* warp_tot, float* tot
 
 // The exact top k of a row by one CTA: the k-th largest key by radix selection (four passes of eight bits), then
 // every key above it and the lowest indices of its equals, into cand[0 .. k).
-__device__ __noinline__ void select_exact(Common& sh, const float* x, int V, int k) {
+__device__ __forceinline__ void select_exact(Common& sh, const float* x, int V, int k) {
   const int tid = threadIdx.x;
   if (tid == 0) {
     sh.prefix = 0;
@@ -175,6 +175,9 @@ __device__ __noinline__ void select_exact(Common& sh, const float* x, int V, int
   __syncthreads();
 }
 
+// (out of line where it is hardly ever needed; inlined, its atomics and loads know their address spaces)
+__device__ __noinline__ void select_exact_cold(Common& sh, const float* x, int V, int k) { select_exact(sh, x, V, k); }
+
 // Reads the CTA's share [lo, hi) of the row (into shared memory where it fits) and returns the thread's maximum and
 // the first index that has it (0x7fffffff: nothing above -inf).
 template <bool STASH>
@@ -199,6 +202,12 @@ __device__ __forceinline__ void read_share(const float* x, int lo, int hi, int c
       }
     }
   }
+}
+
+// The lowest thread of the block for which `hit` holds -> *choice (0xffffffff before).  One atomic per warp: nearly all threads may hit.
+__device__ __forceinline__ void first_thread(bool hit, unsigned* choice) {
+  const unsigned m = __ballot_sync(0xffffffffu, hit);
+  if (m != 0 && (threadIdx.x & 31) == 0) atomicMin(choice, static_cast<unsigned>(threadIdx.x) + __ffs(m) - 1);
 }
 
 // Sorts the gathered candidates and draws among the first k: nucleus, then the inverse CDF.  sh.choice is 0xffffffff.
@@ -241,26 +250,25 @@ __device__ __forceinline__ void draw_sorted(Common& sh, const SampleArgs& a, con
   const float target = u * kept_total;
   // The first candidate whose cumulative probability exceeds the target.  (Not "the one whose interval holds it": intervals formed
   // from the scan overlap, or leave gaps, in their last bit.)
-  if (tid < kk && pj > 0.0f && target < cum) atomicMin(&sh.choice, static_cast<unsigned>(tid));
+  first_thread(tid < kk && pj > 0.0f && target < cum, &sh.choice);
   __syncthreads();
   const unsigned at = sh.choice == 0xffffffffu ? static_cast<unsigned>(kk - 1) : sh.choice;   // none: u * total rounded up to the total
   if (static_cast<unsigned>(tid) == at) a.out[row] = idx;
 }
 
 // The draw inside a chunk [i0, i1) of the row whose exponentials come from `e`: the first one whose cumulative sum exceeds the target, the last
-// one that is not zero where rounding leaves none.
+// one that is not zero where rounding leaves none.  (The sum starts below the target also where the scan has it above: an exponential of zero
+// is never the first to exceed it.)
 template <typename F>
 __device__ __forceinline__ int walk_chunk(int i0, int i1, float before, float target, F e) {
-  float c = before;
-  int pick = i0;
+  float c = fminf(before, target);
   for (int i = i0; i < i1; ++i) {
-    const float v = e(i);
-    if (!(v > 0.0f)) continue;
-    pick = i;
-    c += v;
-    if (target < c) break;
+    c += e(i);
+    if (target < c) return i;
   }
-  return pick;
+  int last = i1 - 1;
+  while (last > i0 && !(e(last) > 0.0f)) --last;
+  return last;
 }
 
 // grid = (cluster, rows)
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
     const float incl = block_scan(part, sh.warp_tot, &total);
     const float target = u * total;
     // the first chunk that reaches beyond the target (the scan's differences overlap, or leave gaps, in their last bit)
-    if (part > 0.0f && target < incl) atomicMin(&sh.choice, static_cast<unsigned>(tid));
+    first_thread(part > 0.0f && target < incl, &sh.choice);
     __syncthreads();
     const unsigned owner = sh.choice;
     if (owner == 0xffffffffu) {
@@ -358,7 +366,8 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
     } else if (owner == static_cast<unsigned>(tid) && tid / cpc == rank) {
       const int i0 = min(tid * chunk, V), i1 = min(i0 + chunk, V);
       const float* e = stash + (tid - rank * cpc) * pitch;
-      a.out[blockIdx.y] = walk_chunk(i0, i1, incl - part, target, [&](int i) { return a.stash ? e[i - i0] : expf((x[i] - gmax) * a.inv_temperature); });
+      a.out[blockIdx.y] = a.stash ? walk_chunk(i0, i1, incl - part, target, [&](int i) { return e[i - i0]; })
+                                  : walk_chunk(i0, i1, incl - part, target, [&](int i) { return expf((x[i] - gmax) * a.inv_temperature); });
     }
     return;
   }
@@ -423,10 +432,77 @@ __global__ void __launch_bounds__(kT, 1) sample_kernel(const SampleArgs a) {
   unsigned n_cand = sh.count;
   __syncthreads();
   if (n_cand > kMaxCand || n_cand < static_cast<unsigned>(k)) {   // (fewer: groups of nothing but NaN)
-    select_exact(sh, x, V, k);
+    select_exact_cold(sh, x, V, k);
     n_cand = static_cast<unsigned>(k);
   }
   draw_sorted(sh, a, x, gmax, u, n_cand, blockIdx.y);
+}
+
+// One CTA per row: what many rows take, which fill the GPU without clusters.  The row is read from L2 as often as needed.
+__global__ void __launch_bounds__(kT, 2) sample_row_kernel(const SampleArgs a) {
+  __shared__ Common sh;
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int V = a.V;
+  const float* x = a.logits + static_cast<size_t>(blockIdx.x) * V;
+  float bv = -INFINITY;
+  int bi = 0x7fffffff;
+#pragma unroll 4
+  for (int i = tid; i < V; i += kT) {
+    const float v = __ldg(x + i);
+    if (v > bv) {
+      bv = v;
+      bi = i;
+    }
+  }
+  best_of_warp(bv, bi);
+  if (lane == 0) {
+    sh.s_val[warp] = bv;
+    sh.s_idx[warp] = bi;
+  }
+  if (tid == 0) sh.choice = 0xffffffffu;
+  __syncthreads();
+  bv = sh.s_val[lane];
+  bi = sh.s_idx[lane];
+  best_of_warp(bv, bi);
+  const float gmax = bv;
+  const int garg = bi == 0x7fffffff ? 0 : bi;   // no logit above -inf
+  if (a.inv_temperature == 0.0f) {
+    if (tid == 0) a.out[blockIdx.x] = garg;
+    return;
+  }
+  const float u = a.uniform[blockIdx.x];
+  if (a.top_k == 0) {
+    const int i0 = min(tid * a.chunk, V), i1 = min(i0 + a.chunk, V);
+    float part = 0.0f;
+    for (int i = i0; i < i1; ++i) part += expf((x[i] - gmax) * a.inv_temperature);
+    float total;
+    const float incl = block_scan(part, sh.warp_tot, &total);
+    const float target = u * total;
+    first_thread(part > 0.0f && target < incl, &sh.choice);
+    __syncthreads();
+    if (sh.choice == 0xffffffffu) {
+      if (tid == 0) a.out[blockIdx.x] = garg;   // u * total rounded up to the total
+    } else if (sh.choice == static_cast<unsigned>(tid)) {
+      a.out[blockIdx.x] = walk_chunk(i0, i1, incl - part, target, [&](int i) { return expf((x[i] - gmax) * a.inv_temperature); });
+    }
+    return;
+  }
+  select_exact(sh, x, V, a.top_k);
+  draw_sorted(sh, a, x, gmax, u, static_cast<unsigned>(a.top_k), blockIdx.x);
+}
+
+// Which kernel: where rows alone fill the GPU, or a row is too short to share, a cluster's exchanges cost more than they save.
+// Measured, one CTA per row / a cluster (us): greedy 8 x 4099 6 / 8, 8 x 32000 12 / 8, 96 x 50257 6 / 10, 256 x 151936 31 / 48; whole row 32 x 8192 5 / 7,
+// 37 x 16384 9 / 14, 32 x 32000 24 / 10, 96 x 50257 20 / 32, 256 x 65536 82 / 85; top 50 64 x 8192 28 / 30 (top 20: 33 / 28), 96 x 8192 28 / 44, 96 x 16384
+// 42 / 47, 64 x 16384 42 / 33, 256 x 32000 108 / 124, 256 x 65536 187 / 135; top 1000 64 x 8192 38 / 51, 37 x 8192 38 / 35, 96 x 50257 67 / 82,
+// 128 x 65536 124 / 110.
+bool RowPerCta(int64_t batch, int64_t vocab, const SampleArgs& a) {
+  if (a.inv_temperature == 0.0f) return vocab <= 16384 || batch >= (vocab <= 65536 ? 96 : 128);
+  if (a.top_k == 0) return vocab <= 8192 || (batch >= 37 && vocab <= 16384) || (batch >= 96 && vocab < 65536) || (batch >= 1024 && vocab <= 65536);
+  if (a.top_k >= 256)
+    return (batch >= (vocab < 2048 ? 112 : 64) && vocab <= 16384) || (batch >= 96 && vocab < 65536) || (batch >= 512 && vocab <= 65536);
+  return (batch >= 80 && vocab <= 8192) || (batch >= 96 && vocab <= 16384) || (batch >= 160 && vocab < 65536);
 }
 
 }  // namespace
@@ -468,6 +544,12 @@ b200_status b200_sample(b200_context* ctx, b200_stream stream, const float* logi
   lc.block = dim3(kT);
   lc.pdl = true;
   cudaError_t e;
+  if (RowPerCta(batch, vocab, a)) {
+    lc.grid = dim3(static_cast<unsigned>(batch));
+    e = Launch(lc, sample_row_kernel, a);
+    if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_sample launch: %s", cudaGetErrorString(e)));
+    return EndLaunch(ctx, "b200_sample");
+  }
   const bool fits4 = kHeader + static_cast<size_t>(kT / 4) * (a.chunk + 1) * sizeof(float) <= static_cast<size_t>(ctx->max_smem_optin);
   const int cluster = batch * 8 <= ctx->sm_count || !fits4 ? 8 : 4;
   const size_t share = static_cast<size_t>(kT / cluster) * (a.chunk + 1) * sizeof(float);

@@ -18,7 +18,7 @@ def _run(p, logits, u, **kw):
     return host(out)
 
 
-@pytest.mark.parametrize("B,V", [(3, 1000), (2, 151936), (5, 4099)])
+@pytest.mark.parametrize("B,V", [(3, 1000), (2, 151936), (5, 4099), (2, 16384), (2, 16385), (96, 30000), (128, 70001)])
 def test_greedy(B, V):
     p = pkg()
     rng = np.random.default_rng(1)
@@ -58,7 +58,10 @@ def test_sampling_matches_the_oracle(kw, V):
 
 @pytest.mark.parametrize("B,V,k", [(3, 50257, 50), (18, 50257, 50), (19, 50257, 50), (2, 1, 1), (3, 700, 700), (3, 1024, 1), (3, 1025, 1024),
                                    (3, 8193, 1000), (2, 1 << 19, 40), (33, 2050, 2), (2, 40000, 0), (33, 4099, 0), (2, 131072, 0),
-                                   (2, 1 << 19, 0), (2, 37, 0)])
+                                   (2, 1 << 19, 0), (2, 37, 0),
+                                   # one CTA per row, and the last batch that clusters take
+                                   (112, 1, 1), (112, 33, 33), (80, 4099, 50), (79, 4099, 50), (96, 16384, 255), (160, 32001, 3), (112, 1025, 1024), (96, 50257, 256),
+                                   (96, 32000, 0), (95, 32000, 0), (37, 16384, 0), (36, 9000, 0)])
 def test_shares_of_a_row(B, V, k):
     """Around the limits of a CTA's share: empty shares, fewer logits than threads, shares beyond shared memory."""
     rng = np.random.default_rng(V + k)
@@ -76,16 +79,22 @@ def test_shares_of_a_row(B, V, k):
 
 
 def test_nan_and_infinite_rows():
-    logits = np.zeros((4, 5000), np.float32)
+    for V in (5000, 40000):
+        _nan_and_infinite_rows(V)
+
+
+def _nan_and_infinite_rows(V):
+    logits = np.zeros((100, V), np.float32)
     logits[0] = -np.inf
     logits[1] = np.nan
     logits[2, 77] = np.inf
     logits[3, ::2] = -np.nan
-    for kw in (dict(temperature=0.0), dict(temperature=1.0), dict(temperature=1.0, top_k=30), dict(temperature=1.0, top_k=1024, top_p=0.5)):
-        got = _run(pkg(), logits, np.full(4, 0.5, np.float32), **kw)
-        assert np.all((got >= 0) & (got < 5000)), kw
-        if kw["temperature"] == 0.0:
-            assert got[2] == 77 and got[0] == 0
+    for B in (4, 100):
+        for kw in (dict(temperature=0.0), dict(temperature=1.0), dict(temperature=1.0, top_k=30), dict(temperature=1.0, top_k=1024, top_p=0.5)):
+            got = _run(pkg(), logits[:B], np.full(B, 0.5, np.float32), **kw)
+            assert np.all((got >= 0) & (got < V)), kw
+            if kw["temperature"] == 0.0:
+                assert got[2] == 77 and got[0] == 0
 
 
 def test_refusals():
