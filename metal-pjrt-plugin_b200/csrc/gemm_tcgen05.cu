@@ -922,25 +922,36 @@ cudaError_t LaunchFor(int out_dtype, const CUtensorMap& ma, const CUtensorMap& m
   return LaunchTc<BN, CG, __half, kWide>(ma, mb, a, idesc, grid, stream);
 }
 
-// The quantised product: tiles of 128 x 256 or 128 x 128 and the split of K by the same kind of cost model as RunTcgen05.
-constexpr double kWidenStep256 = 0.40, kWidenStep128 = 0.25;   // us per 64-deep step of a tile
+struct TilePlan {
+  int bn = 256, group = 1, split = 1;   // columns of a tile, CTAs of a tile, CTAs along K
+  double us = 1e30;
+};
+
+// The quantised product: tiles of 128 x 256 or 128 x 128 and the split of K by the same kind of cost model as PlanDense.
+constexpr double kWidenStep256 = 0.40, kWidenStep128 = 0.25;   // per 64-deep step of a tile, relative to the epilogues'
 template <int WQ>
-b200_status RunQuantised(b200_context* ctx, cudaStream_t stream, const CUtensorMap& ma, const b200_qmm_params* p, TcArgs a, int out_dtype) {
-  const int64_t k_iters = a.k / BK;
-  int bn = 256, split = 1;
-  double best = 1e30;
+TilePlan PlanQuantised(const b200_context* ctx, int64_t m, int64_t n, int64_t k, int out_dtype) {
+  const int64_t k_iters = k / BK;
+  TilePlan p;
   for (int cand : {256, 128}) {
     const double t_iter = cand == 256 ? kWidenStep256 : kWidenStep128, epi = cand == 256 ? 4.0 : 2.3;
-    const int64_t tiles = CeilDiv(a.m, BM) * CeilDiv(a.n, cand);
+    const int64_t tiles = CeilDiv(m, BM) * CeilDiv(n, cand);
     const double whole = static_cast<double>(CeilDiv(tiles, ctx->sm_count)) * std::max(k_iters * t_iter, epi) + epi;
-    if (whole < best) best = whole, bn = cand, split = 1;
+    if (whole < p.us) p.us = whole, p.bn = cand, p.split = 1;
     for (int sp = 2; sp <= 8 && cand == 128; sp *= 2) {
       if (tiles * sp > ctx->sm_count || k_iters / sp < 4) break;
       if (tiles > ResidentClustersFor<128, 1, WQ>(out_dtype, sp)) continue;
       const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 1.5 + epi;
-      if (cost < best) best = cost, bn = cand, split = sp;
+      if (cost < p.us) p.us = cost, p.bn = cand, p.split = sp;
     }
   }
+  return p;
+}
+
+template <int WQ>
+b200_status RunQuantised(b200_context* ctx, cudaStream_t stream, const CUtensorMap& ma, const b200_qmm_params* p, TcArgs a, int out_dtype) {
+  const TilePlan plan = PlanQuantised<WQ>(ctx, a.m, a.n, a.k, out_dtype);
+  const int bn = plan.bn, split = plan.split;
   a.split = split;
   a.tiles_n = static_cast<int>(CeilDiv(a.n, bn));
   a.stage_bytes = (a.a_rows + bn) * BK * 2;
@@ -955,6 +966,46 @@ b200_status RunQuantised(b200_context* ctx, cudaStream_t stream, const CUtensorM
                                   : LaunchFor<128, 1, WQ>(out_dtype, ma, mb, a, idesc, grid, stream);
   if (e != cudaSuccess) return Stick(ctx, Fail(B200_INTERNAL, "b200_qmm (tcgen05) launch: %s", cudaGetErrorString(e)));
   return EndLaunch(ctx, "b200_qmm (tcgen05)");
+}
+
+int ARows(int64_t m, int ta) { return ta ? BM : static_cast<int>(std::min<int64_t>(BM, CeilDiv(m, 8) * 8)); }
+
+// Tile shape and K split by a small cost model (microseconds); tiles run in waves over
+// the SMs (256 x 256 tiles over pairs of SMs).  When the tiles leave SMs idle, a cluster of
+// 2/4/8 CTAs splits one tile's K loop (a serial chain on one SM otherwise) and adds the partial
+// tiles through distributed shared memory, for a fixed cost of the cluster barriers and the extra pass.
+// straddle: rows of D whose 16-byte pieces are not aligned.
+TilePlan PlanDense(const b200_context* ctx, int64_t m, int64_t n, int64_t k, int64_t batch, int ta, int out_dtype, bool straddle) {
+  const int64_t k_iters = CeilDiv(k, BK);
+  const int a_rows = ARows(m, ta);
+  // A k step moves a_rows x 64 of A and bn x 64 of B into an SM at about 0.1 MB/us; the MMAs of a 256-wide
+  // tile take 0.27 us.  epi: one tile's epilogue and stores, overlapped with the next tile's loop (measured with K = 64,
+  // 8192 x 8192: 43 / 65 / 74 us for the three shapes, about the write limit of HBM; rows whose 128-byte pieces straddle
+  // lines take twice as long).
+  auto waves_cost = [&](int64_t tiles, int64_t slots, double t_iter, double epi) {
+    return static_cast<double>(CeilDiv(tiles, slots)) * std::max(k_iters * t_iter, epi) + epi;
+  };
+  TilePlan p;
+  {
+    const int pairs = ResidentClustersFor<256, 2>(out_dtype, 1);
+    const int64_t tiles = CeilDiv(m, 2 * BM) * CeilDiv(n, 256) * batch;
+    if (pairs > 0 && m > BM) p.us = waves_cost(tiles, pairs, 0.39, straddle ? 6.6 : 3.0), p.group = 2;
+  }
+  for (int cand : {128, 64}) {
+    // 64 columns are 128-byte pieces of B's rows, which stream at about 0.8 of the rate of 256-byte ones
+    const double t_iter = (a_rows + cand) * (BK * 2) * (cand == 64 ? 1.25e-5 : 1e-5), epi = cand == 128 ? (straddle ? 4.5 : 2.3) : (straddle ? 3.4 : 1.3);
+    const int64_t tiles = CeilDiv(m, BM) * CeilDiv(n, cand) * batch;
+    const double whole = waves_cost(tiles, ctx->sm_count, t_iter, epi);
+    if (whole < p.us) p.us = whole, p.bn = cand, p.group = 1, p.split = 1;
+    for (int sp = 2; sp <= 8; sp *= 2) {
+      if (tiles * sp > ctx->sm_count || k_iters / sp < 4) break;
+      const int resident = cand == 128 ? ResidentClustersFor<128, 1>(out_dtype, sp) : ResidentClustersFor<64, 1>(out_dtype, sp);
+      if (tiles > resident) continue;   // a second wave of clusters would double the time
+      const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 1.5 + epi;
+      if (cost < p.us) p.us = cost, p.bn = cand, p.group = 1, p.split = sp;
+    }
+  }
+  return p;
 }
 
 }  // namespace
@@ -981,42 +1032,10 @@ bool Tcgen05Supports(const b200_gemm_params* p, const b200_epilogue* epi) {
 b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_params* p, const b200_epilogue* epi) {
   const int ta = p->a.transpose, tb = p->b.transpose;
   const int64_t m = p->m, n = p->n, k = p->k, batch = p->batch;
-  // Tile shape and K split by a small cost model (microseconds); tiles run in waves over
-  // the SMs (256 x 256 tiles over pairs of SMs).  When the tiles leave SMs idle, a cluster of
-  // 2/4/8 CTAs splits one tile's K loop (a serial chain on one SM otherwise) and adds the partial
-  // tiles through distributed shared memory, for a fixed cost of the cluster barriers and the extra pass.
-  const int64_t k_iters = CeilDiv(k, BK);
-  const int a_rows = ta ? BM : static_cast<int>(std::min<int64_t>(BM, CeilDiv(m, 8) * 8));
-  // A k step moves a_rows x 64 of A and bn x 64 of B into an SM at about 0.1 MB/us; the MMAs of a 256-wide
-  // tile take 0.27 us.  epi: one tile's epilogue and stores, overlapped with the next tile's loop (measured with K = 64,
-  // 8192 x 8192: 43 / 65 / 74 us for the three shapes, about the write limit of HBM; rows whose 128-byte pieces straddle
-  // lines take twice as long).
-  const int out_size = DtypeSize(p->c.dtype);
-  const bool straddle = (p->c.ld * out_size) % 16 != 0 || !Aligned(p->c.ptr, 16);
-  auto waves_cost = [&](int64_t tiles, int64_t slots, double t_iter, double epi) {
-    return static_cast<double>(CeilDiv(tiles, slots)) * std::max(k_iters * t_iter, epi) + epi;
-  };
-  int bn = 256, group = 1, split = 1;
-  double best = 1e30;
-  {
-    const int pairs = ResidentClustersFor<256, 2>(p->c.dtype, 1);
-    const int64_t tiles = CeilDiv(m, 2 * BM) * CeilDiv(n, 256) * batch;
-    if (pairs > 0 && m > BM) best = waves_cost(tiles, pairs, 0.39, straddle ? 6.6 : 3.0), group = 2;
-  }
-  for (int cand : {128, 64}) {
-    // 64 columns are 128-byte pieces of B's rows, which stream at about 0.8 of the rate of 256-byte ones
-    const double t_iter = (a_rows + cand) * (BK * 2) * (cand == 64 ? 1.25e-5 : 1e-5), epi = cand == 128 ? (straddle ? 4.5 : 2.3) : (straddle ? 3.4 : 1.3);
-    const int64_t tiles = CeilDiv(m, BM) * CeilDiv(n, cand) * batch;
-    const double whole = waves_cost(tiles, ctx->sm_count, t_iter, epi);
-    if (whole < best) best = whole, bn = cand, group = 1, split = 1;
-    for (int sp = 2; sp <= 8; sp *= 2) {
-      if (tiles * sp > ctx->sm_count || k_iters / sp < 4) break;
-      const int resident = cand == 128 ? ResidentClustersFor<128, 1>(p->c.dtype, sp) : ResidentClustersFor<64, 1>(p->c.dtype, sp);
-      if (tiles > resident) continue;   // a second wave of clusters would double the time
-      const double cost = static_cast<double>(CeilDiv(k_iters, sp)) * t_iter + 1.5 + epi;
-      if (cost < best) best = cost, bn = cand, group = 1, split = sp;
-    }
-  }
+  const int a_rows = ARows(m, ta);
+  const bool straddle = (p->c.ld * DtypeSize(p->c.dtype)) % 16 != 0 || !Aligned(p->c.ptr, 16);
+  const TilePlan plan = PlanDense(ctx, m, n, k, batch, ta, p->c.dtype, straddle);
+  const int bn = plan.bn, group = plan.group, split = plan.split;
   TcArgs a;
   a.a_rows = a_rows;
   a.stage_bytes = (a_rows + bn / group) * BK * 2;
@@ -1070,6 +1089,27 @@ b200_status RunTcgen05(b200_context* ctx, cudaStream_t stream, const b200_gemm_p
 bool QuantisedGemmSupports(const b200_qmm_params* p) {
   const int64_t ldx = p->ldx ? p->ldx : p->K;
   return p->bits != 16 && Encoder() != nullptr && Aligned(p->x, 16) && ldx % 8 == 0 && CeilDiv(p->M, BM) * CeilDiv(p->N, 128) <= INT32_MAX;
+}
+
+// Whether dequantising panels of `panel` weight rows and multiplying by those is the faster form: both times estimated (microseconds, cold caches),
+// fitted to 144 products of each format, 64 to 8192 rows, at nine shapes between 1024 x 1024 and 24576 x 4096; the estimates are within 7 %
+// of what was measured on average, and the form they choose within 0.5 % of the better one (16 % at most).  Dequantising costs per weight, sequential int4 at
+// memory speed, the others by a general kernel; the direct form widens the weights again for every 128 rows of x.  Measured, direct / panels (us):
+// int4 256 x 4096 -> 4096 31 / 33, 320 rows 41 / 35; 512 x 4096 -> 24576 158 / 167, 640 rows 202 / 169; 256 x 12288 -> 4096 67 / 76, 320 rows
+// 108 / 88; int8 per channel 1536 x 4096 -> 4096 118 / 117, 2048 x 4096 -> 24576 652 / 637, 4096 rows 1252 / 955; split-half int4 4096 x 4096 -> 24576 1123 / 1114.
+bool PanelsAreFaster(const b200_context* ctx, const b200_qmm_params* p, int64_t panel) {
+  const int out = p->epilogue == B200_QMM_OUT_F32_RAW ? B200_F32 : B200_BF16;
+  const bool seq = p->bits == 4 && p->nibble_order == 0;
+  const TilePlan d = p->bits == 8 ? PlanQuantised<kQ8>(ctx, p->M, p->N, p->K, out)
+                                  : (seq ? PlanQuantised<kQ4Seq>(ctx, p->M, p->N, p->K, out) : PlanQuantised<kQ4Half>(ctx, p->M, p->N, p->K, out));
+  const int64_t waves = d.split > 1 ? 1 : CeilDiv(CeilDiv(p->M, BM) * CeilDiv(p->N, d.bn), ctx->sm_count);
+  const double step = d.bn == 256 ? 0.78 : 0.50, epi = d.bn == 256 ? 4.0 : 2.3;
+  const double direct = waves * std::max(CeilDiv(p->K / BK, d.split) * step, 2.0) + epi + 8.0 + (d.split > 1 ? 4.5 : 0.0);
+  double gemm = 0.0;
+  for (int64_t r = 0; r < p->N; r += panel) gemm += PlanDense(ctx, p->M, std::min(panel, p->N - r), p->K, 1, 0, out, false).us;
+  const double weights = static_cast<double>(p->N) * p->K * 1e-6 * (seq ? 0.52 : (p->bits == 4 ? 5.67 : 3.82));
+  const double panels = 0.82 * gemm + weights + 12.5 * CeilDiv(p->N, panel);
+  return panels < direct;
 }
 
 b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {

@@ -4,7 +4,7 @@
 //     (gemm_tcgen05.cu): no bf16 copy exists, but every row of 128 x tiles widens them again;
 //   * the weights are dequantised panel by panel into bf16 scratch and each panel goes through the general GEMM
 //     (PanelsAreFaster says when, and rows of x that TMA cannot read).  A panel is at most 96 MB (or 256 rows), so that it stays in
-//     the 126 MB L2: 32 MB panels gave GEMMs of less than a wave of tiles (int4 512 x 12288 -> 4096: 136 us, now 87).  The scratch
+//     the 126 MB L2: 32 MB panels gave GEMMs of less than a wave of tiles (int4 512 x 12288 -> 4096: 147 us, now 88).  The scratch
 //     is stream-ordered memory of the context's pool: calls on several streams each have their own, and a graph owns its.
 #include <algorithm>
 
@@ -16,11 +16,6 @@ using namespace b200;
 namespace {
 
 constexpr int64_t kPanelBytes = 96ll << 20;
-
-// Many rows of x pay for the copy.  Only sequential int4 has a kernel that writes it at memory speed.  us for the
-// direct form against panels, 4096 -> 24576 and 12288 -> 4096 with cold caches: 256 rows 107 / 61 against 125 / 73, 512 rows
-// 156 / 102 against 150 / 87 (back to back 4096 -> 24576: 154 against 170), 1024 rows 285 / 154 against 204 / 104.
-bool PanelsAreFaster(const b200_qmm_params* p) { return p->bits == 4 && p->nibble_order == 0 && p->M > 512; }
 
 // Sequential int4 in groups of 64: one thread per 8 inputs (one word), 16-byte stores.
 __global__ void dequant_int4_seq_kernel(const uint32_t* q, const __nv_bfloat16* scale, const __nv_bfloat16* bias, uint4* out,
@@ -111,6 +106,7 @@ namespace b200 {
 
 // gemm_tcgen05.cu
 bool QuantisedGemmSupports(const b200_qmm_params* p);
+bool PanelsAreFaster(const b200_context* ctx, const b200_qmm_params* p, int64_t panel);
 b200_status RunQuantisedGemm(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p);
 
 b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_params* p) {
@@ -121,15 +117,17 @@ b200_status QmmManyRows(b200_context* ctx, cudaStream_t stream, const b200_qmm_p
     return Fail(B200_UNIMPLEMENTED, "b200_qmm: above 32 rows the output is bf16, bf16 + residual, or raw f32");
   const int64_t M = p->M, N = p->N, K = p->K;
   const int64_t ldo = p->ldo ? p->ldo : N;
-  const bool direct_ok = QuantisedGemmSupports(p);
-  bool direct = direct_ok && !PanelsAreFaster(p);
   // bf16 weights need no scratch: one GEMM over the whole matrix
   int64_t panel = N;
-  void* ws = nullptr;
-  if (p->bits != 16 && !direct) {
+  if (p->bits != 16) {
     // panels of equal height: a short last one is less than a wave of tiles
     const int64_t most = std::max<int64_t>(256, kPanelBytes / (2 * K) / 256 * 256);
     panel = std::min(CeilDiv(CeilDiv(N, CeilDiv(N, most)), 256) * 256, N);
+  }
+  const bool direct_ok = QuantisedGemmSupports(p);
+  bool direct = direct_ok && !PanelsAreFaster(ctx, p, panel);
+  void* ws = nullptr;
+  if (p->bits != 16 && !direct) {
     const size_t need = static_cast<size_t>(panel) * K * 2;
     const cudaError_t e = cudaMallocFromPoolAsync(&ws, need, ctx->pool, stream);
     if (e != cudaSuccess) {

@@ -53,6 +53,16 @@ def test_batched_edges(n, k, kind):
         _check(p, m, n, k, kind)
 
 
+@pytest.mark.parametrize("kind", ["int4", "int4_half", "int8", "int8_g64"])
+@pytest.mark.parametrize("m,n,k", [(320, 4096, 4096), (640, 1031, 1024), (8200, 1026, 1088)])
+def test_panels(m, n, k, kind):
+    """Many rows: dequantised panels (of the other formats from thousands of rows on), or weights widened in the GEMM, as the times say."""
+    p = pkg()
+    _check(p, m, n, k, kind)
+    if m < 1000:
+        _check(p, m, n, k, kind, form="residual")
+
+
 @pytest.mark.parametrize("kind", ["int4", "int8", "int8_g64"])
 @pytest.mark.parametrize("m", [9, 24, 40])
 def test_batched_forms(m, kind):
