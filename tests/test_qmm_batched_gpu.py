@@ -22,19 +22,21 @@ def _weight(p, kind, n, k, seed):
     return q, p.qwen3.dequantize(q, torch.float32).double()
 
 
-def _check(p, m, n, k, kind, form="plain", pad=0):
+def _check(p, m, n, k, kind, form="plain", pad=0, shift=0):
+    """pad: elements between the rows of x; shift: elements before its first."""
     import torch
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     w, w64 = _weight(p, kind, n, k, m)
     cols = 2 * k if form == "silu" else k
-    x = torch.randn((m, cols + pad), generator=g, device="cuda").to(torch.bfloat16)[:, :cols]
+    x = torch.randn((m * (cols + pad) + shift,), generator=g, device="cuda").to(torch.bfloat16)[shift:].view(m, cols + pad)[:, :cols]
     a = x.double()
     if form == "silu":      # bf16 roundings of the sigmoid, gate * sigmoid and the product
         gate, up = x[:, :k].float(), x[:, k:].float()
         sig = torch.sigmoid(gate).to(torch.bfloat16).float()
         a = ((gate * sig).to(torch.bfloat16).float() * up).to(torch.bfloat16).double()
     res = torch.randn((m, n), generator=g, device="cuda").to(torch.bfloat16) if form == "residual" else None
-    got = p.qwen3.linear(x if pad == 0 else x.contiguous(), w, residual=res, silu_mul=form == "silu").double()
+    assert x.data_ptr() % 16 == 2 * shift % 16 and (m == 1 or x.stride(0) == cols + pad)
+    got = p.qwen3.linear(x, w, residual=res, silu_mul=form == "silu").double()
     v, mag = a @ w64.T, a.abs() @ w64.abs().T
     want = v + (res.double() if res is not None else 0)
     # results are rounded to bf16 (2^-8 in all for two roundings); sums of k f32 terms; above 32 rows the weights are bf16 (2^-9)
@@ -51,6 +53,17 @@ def test_batched_edges(n, k, kind):
     p = pkg()
     for m in (9, 16, 17, 32, 33, 129, 513):
         _check(p, m, n, k, kind)
+
+
+@pytest.mark.parametrize("kind", ["int4", "int4_half", "int8", "int8_g64", "bf16"])
+@pytest.mark.parametrize("pad,shift", [(1, 0), (3, 0), (8, 0), (0, 1), (0, 8), (5, 3)])
+def test_rows_that_allow_no_wide_loads(pad, shift, kind):
+    """x whose rows or first element are not 16-byte aligned (or just are): staged element by element, or copied into aligned rows."""
+    p = pkg()
+    for m in (9, 17, 32, 33, 129):
+        _check(p, m, 257, 1088, kind, pad=pad, shift=shift)
+        _check(p, m, 130, 576, kind, form="residual", pad=pad, shift=shift)
+    _check(p, 24, 130, 576, kind, form="silu", pad=pad, shift=shift)
 
 
 @pytest.mark.parametrize("kind", ["int4", "int4_half", "int8", "int8_g64"])
