@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qmm_mid_kernel(const __grid
 
   int s = 0;
   uint32_t parity = 0;
-  bool dead = false;   // a bounded wait gave up
-  for (int tile = tile0; tile < a.tiles && !dead; tile += tile_step) {
+  int flying = 0;   // a bounded wait gave up: the boxes that are still to land
+  for (int tile = tile0; tile < a.tiles && flying == 0; tile += tile_step) {
     const int n0 = tile * kRows;
     float acc[2][MB][4];
 #pragma unroll
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qmm_mid_kernel(const __grid
     for (int bx = 0; bx < boxes; ++bx) {
       if (!mbar_wait_bounded(&bars[warp][s], parity)) {
         report_timeout(a.status, 200 + s);
-        dead = true;
+        flying = min(a.stages, boxes - bx + boxes * ((a.tiles - 1 - tile) / tile_step));   // (fetches run a whole ring ahead)
         break;
       }
 #pragma unroll
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qmm_mid_kernel(const __grid
       fetch();
       if (++s == a.stages) s = 0, parity ^= 1;
     }
-    if (dead) break;
+    if (flying > 0) break;
 #pragma unroll
     for (int rt = 0; rt < 2; ++rt)
 #pragma unroll
@@ -326,6 +326,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) qmm_mid_kernel(const __grid
       scales(tile + tile_step);
       __syncwarp();
     }
+  }
+  // No box may land in this CTA's shared memory once it is gone (one more wait that runs out ends this).
+  for (; flying > 0; --flying) {
+    if (!mbar_wait_bounded(&bars[warp][s], parity)) break;
+    if (++s == a.stages) s = 0, parity ^= 1;
   }
 }
 
