@@ -1,7 +1,7 @@
 // Measurement only: how many SM cycles one tcgen05.mma costs, by shape.  One CTA, one issuing
 // thread, `count` instructions back to back, then a commit and a bounded wait on its mbarrier.
-// The answer on B200 (about 194 cycles whatever N, M, kind or A source) is why the int4 product
-// for a handful of rows stays on mma.sync (see qmm_tc.cu).
+// It issues from a thread picked by its index, as qmm_tc.cu does: about 194 cycles whatever N, M, kind or A source.  From
+// a lane picked by elect.sync the same instructions take 48 to 127 (gemm_tcgen05.cu), which this probe does not show.
 #include "common.cuh"
 
 using namespace b200;

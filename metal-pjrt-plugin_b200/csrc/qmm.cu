@@ -1,4 +1,4 @@
-// Weight-only quantised matmul for few rows (M <= 32), the decode path:
+// Weight-only quantised matmul for few rows (M <= 8, and up to 32 as below), the decode path:
 //   out[M, N] = x[M, K] . dequant(W)[N, K]^T
 // The reference has no kernel for this; XLA turns its _matvec_int4/_matvec_int8
 // (examples/llm/qwen3.py:233-267) into generic row reductions.  The math kept

@@ -1,14 +1,11 @@
 // int4-g64 dequant-matmul for up to 8 rows of x on the 5th-generation tensor cores
 // (≙ _matvec_int4 / dequantize + dot of the reference, examples/llm/qwen3.py:199-267).
 //
-// Status: an alternative route, taken only with B200_QMM_TC=1.  It is correct (the parity tests
-// pass on it) but slower than the mma.sync kernel for these shapes, for a reason measured on the
-// device: one tcgen05.mma costs ~194 SM cycles whatever its N (16 ... 256), M (64, 128), operand
-// kind (f8f6f4, f16) or A source (shared or tensor memory).  With the weights on the M side an
-// instruction covers 128 rows x 32 inputs = 2 KB of nibbles, so an SM cannot stream more than
-// 2 KB / 194 cycles = 10.5 B/cycle: 2.95 TB/s over 148 SMs at 1.9 GHz, below what the mma.sync
-// kernel reaches (3.5 TB/s on the 24576 x 4096 projection).  The tensor core only pays once the
-// batch fills the instruction's N (hundreds of columns).
+// Status: an alternative route, taken only with B200_QMM_TC=1 or b200_qmm_force_route 2.  It is correct (the parity tests
+// pass on it) but slower than the mma.sync kernel: 37 us against 17 on the 24576 x 4096 projection, one row.  Its MMAs
+// are issued by a thread picked by its index, at ~194 SM cycles each whatever their shape; 2 KB of nibbles per instruction
+// (128 rows x 32 inputs) then caps an SM at 10.5 B/cycle.  That is the cost of this form of issue: the dense GEMM's, from a lane
+// picked by elect.sync, take 48 to 127 cycles (gemm_tcgen05.cu).  What this kernel would do with one has not been measured.
 //
 // The idea: with mma.sync the nibbles have to be widened to bf16 in registers (4 two-cycle logic
 // operations per 8 weights, plus the fragment loads and the MMA issue), and that ALU work, not

@@ -13,15 +13,15 @@
 //
 // Bound by latency: one pass over the logits is 3 us of HBM for 32 rows of 151936, and one CTA per row
 // (which re-read its row from L2 six to ten times and met on single histogram counters) took 158 us for that.
-// A cluster of CTAs takes a row (many or short rows: one CTA each, see RowPerCta).  Each reads its share once into shared memory, where all later passes run;
-// the CTAs exchange maxima, thresholds and candidates by stores into each other's shared memory.
+// A cluster of CTAs takes a row (many or short rows: one CTA each, see RowPerCta).  Each reads its share once into shared
+// memory, where all later passes run; the CTAs exchange maxima, thresholds and candidates by stores into each other's shared memory.
 //   top-k   every thread's maximum is one of kT x cluster groups, so the k-th largest maximum is a lower bound
 //           of the k-th largest logit, and hardly more than k logits reach it: those are gathered in the first
 //           CTA and sorted there.  The bound is found by bisection over the maxima, which every CTA holds.
 //           More than kMaxCand candidates (long runs of equal logits) take an exact radix selection instead.
 //   all     the row's exponentials are formed in place; 1024 contiguous chunks are summed one thread each, in
 //           the order in which the draw then walks the chosen chunk.
-// 32 x 151936, top-k 20 + top-p: 158 -> 17 us; 21 x 128256, all: 65 -> 17 us.
+// Against one CTA per row: 32 x 151936, top-k 20 + top-p 158 -> 17 us, whole row 67 -> 20; 32 x 32000, whole row 28 -> 10.
 #include <algorithm>
 
 #include <cooperative_groups.h>

@@ -15,7 +15,8 @@ from .context import default_context
 from .rows import rms_norm  # noqa: F401  (qwen3.py:294-297)
 
 GROUP = 64
-ROWS_MAX = 32  # the streaming kernel's row limit (the reference's is 4, qwen3.py:215)
+ROWS_MAX = 32  # rows of the decode kernels, which take fused inputs and keep f32 weights; more go to the tensor-core GEMM
+#               (the reference's limit is 4, qwen3.py:215)
 
 
 def _torch():
@@ -100,7 +101,8 @@ def interleave_gate_up(w, ctx=None):
 def linear(x, w, residual=None, out_f32=False, rms_gain=None, eps=1e-6, silu_mul=False, silu_pair=False, ctx=None,
            stream=None):
     """≙ linear (qwen3.py:218-230): x @ w.T for an [out, in] weight, bf16 or
-    quantised, up to ROWS_MAX rows; result in x's dtype (bf16).  `residual`
+    quantised; result in x's dtype (bf16).  Above ROWS_MAX rows the
+    weights are rounded to bf16 first.  `residual`
     fuses the x + linear(...) of the decoder layer; out_f32 gives the LM head's
     f32 logits.  rms_gain fuses linear(rms_norm(x, rms_gain, eps), w) (up to 8
     rows); silu_mul fuses linear(silu(gate) * up, w) for x = [gate | up]."""
